@@ -60,8 +60,8 @@ struct ctfp_plan {
     size_t fs_raw_elems = 0;
     float* d_fs_L = nullptr;
     size_t fs_L_elems = 0;
-    // corner-expanded adjoint accumulators (allocated on first backward)
-    float4* d_gexp[kMaxM] = {};
+    float* d_gcol = nullptr;  // adjoint accumulators (grown on demand)
+    size_t gcol_elems = 0;
     // staging for ctfp_forward_host
     float* h2d_vol[kMaxM] = {};
     float* d2h_I = nullptr;
@@ -397,15 +397,20 @@ ctfp_status prepare_volumes(ctfp_plan* p, const float* const* volumes, cudaStrea
     return CTFP_OK;
 }
 
-// Zeroed corner-expanded accumulators for one adjoint launch.
-ctfp_status prepare_expanded(ctfp_plan* p, MarchParams& prm, cudaStream_t st)
+// The adjoint of views [prm.view0, prm.view0 + prm.n_views) into prm.gvol:
+// zeroed accumulators, scatter, fold.
+ctfp_status scatter_and_fold(ctfp_plan* p, MarchParams prm, bool from_gL, cudaStream_t s)
 {
-    const size_t n = expanded_elems(p->gp);
-    for (int m = 0; m < p->M; m++) {
-        if (!p->d_gexp[m]) CTFP_CUDA(cudaMalloc(&p->d_gexp[m], n * sizeof(float4)));
-        CTFP_CUDA(cudaMemsetAsync(p->d_gexp[m], 0, n * sizeof(float4), st));
-        prm.gexp[m] = p->d_gexp[m];
+    if (accum_fits(p->gp.nx, p->gp.ny, p->gp.nz)) {  // else prm.gcol stays null: no accumulators
+        prm.sets = accum_set_count(p->gp, prm.n_views, p->M);
+        prm.set_floats = accum_floats(p->gp.nx, p->gp.ny, p->gp.nz, p->M);
+        const ctfp_status st = ensure_scratch(p->d_gcol, p->gcol_elems, prm.set_floats * prm.sets);
+        if (st != CTFP_OK) return st;
+        prm.gcol = p->d_gcol;
+        CTFP_CUDA(cudaMemsetAsync(prm.gcol, 0, sizeof(float) * prm.set_floats * prm.sets, s));
     }
+    CTFP_CUDA(launch_backward(prm, p->M, p->interp, from_gL, p->shape, s));
+    CTFP_CUDA(launch_fold(prm, p->M, s));
     return CTFP_OK;
 }
 
@@ -495,6 +500,7 @@ ctfp_status ctfp_plan_create(const ctfp_geometry* g, int32_t n_materials, int32_
     gp.pHalfX = info.pHalfX; gp.pHalfY = info.pHalfY; gp.pHalfZ = info.pHalfZ;
     gp.pSizeX = info.pSizeX; gp.pSizeY = info.pSizeY; gp.pSizeZ = info.pSizeZ;
     gp.rpSizeX = 1.0f / info.pSizeX; gp.rpSizeY = 1.0f / info.pSizeY; gp.rpSizeZ = 1.0f / info.pSizeZ;
+    gp.qx = 1.0 / (double)info.pSizeX; gp.qy = 1.0 / (double)info.pSizeY; gp.qz = 1.0 / (double)info.pSizeZ;
     std::vector<double2> trig((size_t)g->projNum);
     std::vector<float2> trigf((size_t)g->projNum);
     for (int64_t k = 0; k < g->projNum; k++) {
@@ -552,7 +558,7 @@ ctfp_status ctfp_plan_destroy(ctfp_plan* p)
     cudaFree(p->d_I0);
     cudaFree(p->d_count);
     for (int m = 0; m < kMaxM; m++) cudaFree(p->h2d_vol[m]);
-    for (int m = 0; m < kMaxM; m++) cudaFree(p->d_gexp[m]);
+    cudaFree(p->d_gcol);
     cudaFree(p->d_occ);
     cudaFree(p->d_status);
     for (cudaEvent_t& e : p->chunk_done)
@@ -854,12 +860,7 @@ static ctfp_status backward_range(ctfp_plan* p, const float* L_ckpt, const float
     prm.out_view0 = compact ? (int)view0 : 0;
     for (int m = 0; m < p->M; m++) prm.gvol[m] = g_volumes[m];
     if (n_views == 0) return CTFP_OK;
-    cudaStream_t s = (cudaStream_t)stream;
-    ctfp_status st = prepare_expanded(p, prm, s);
-    if (st != CTFP_OK) return st;
-    CTFP_CUDA(launch_backward(prm, p->M, p->interp, false, p->shape, s));
-    CTFP_CUDA(launch_fold(prm, p->M, s));
-    return CTFP_OK;
+    return scatter_and_fold(p, prm, false, (cudaStream_t)stream);
 }
 
 ctfp_status ctfp_backward(ctfp_plan* p, const float* L_ckpt, const float* gI, const float* gIAbsorb,
@@ -884,12 +885,7 @@ ctfp_status ctfp_line_integrals_adjoint(ctfp_plan* p, const float* gL, float* co
     MarchParams prm = base_params(p);
     prm.Lin = gL;
     for (int m = 0; m < p->M; m++) prm.gvol[m] = g_volumes[m];
-    cudaStream_t s = (cudaStream_t)stream;
-    ctfp_status st = prepare_expanded(p, prm, s);
-    if (st != CTFP_OK) return st;
-    CTFP_CUDA(launch_backward(prm, p->M, p->interp, true, p->shape, s));
-    CTFP_CUDA(launch_fold(prm, p->M, s));
-    return CTFP_OK;
+    return scatter_and_fold(p, prm, true, (cudaStream_t)stream);
 }
 
 ctfp_status ctfp_sample_volume(const float* volume, int64_t nx, int64_t ny, int64_t nz, int32_t interp,

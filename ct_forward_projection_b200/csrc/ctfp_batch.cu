@@ -15,7 +15,7 @@
 // checkpoint) and the fused forward + loss + adjoint, which for every ray
 // marches, forms I, the loss term (log I - log I_target)^2 and its gradient,
 // recomputes the spectral weights, and marches again scattering into the
-// corner-expanded accumulators; a fold kernel then adds the accumulators into
+// accumulators of ctfp_column.cuh; a fold kernel then adds the accumulators into
 // the gradients.
 #include <algorithm>
 #include <cstring>
@@ -26,6 +26,7 @@
 
 #include "../../include/ctfp.h"
 #include "ctfp_axis.cuh"
+#include "ctfp_column.cuh"
 #include "ctfp_kernels.cuh"
 
 namespace ctfp {
@@ -88,7 +89,9 @@ struct ItemDesc {
     float* L;
     const float* I_target;
     float* gvol[kMaxM];
-    float4* gexp[kMaxM];
+    float* gcol;       // accumulators of every material (ctfp_column.cuh); null: gvol takes the sums directly
+    int sets, set_groups;  // sets of accumulators, and the view groups that sum into one (accum_sets)
+    size_t set_floats;
     float* loss;       // device scalar accumulated with atomicAdd
 };
 
@@ -162,8 +165,7 @@ __device__ __forceinline__ Corner batch_corner(const ItemDesc& it, const RaySeg&
 // in TEXTURE mode the hardware tex3D at the reference's FP32 coordinates (as
 // k_forward).
 template <int M, int MODE, bool AXIS>
-__device__ __forceinline__ void batch_march(const ItemDesc& it, const ItemTex<M>& tx, const RaySeg& s,
-                                            const RayRef32& r, int p, int v, int u, float* L)
+__device__ __forceinline__ void batch_march(const ItemDesc& it, const ItemTex<M>& tx, int p, int v, int u, float* L)
 {
     if (AXIS && MODE != INTERP_TEXTURE) {
         const OccView none{nullptr, 0, 0, 0, 0, 0, 0};
@@ -172,6 +174,9 @@ __device__ __forceinline__ void batch_march(const ItemDesc& it, const ItemTex<M>
         else march_ray_axis<M, AM, 1, false>(it.g, tx.x, tx.y, none, p, v, u, L);
         return;
     }
+    const RaySeg s = ray_segment(it.g, p, v, u);
+    RayRef32 r;
+    if (MODE != INTERP_TRILINEAR) r = ray_ref32(it.g, p, v, u);
     float acc[M], cmp[M];
 #pragma unroll
     for (int m = 0; m < M; m++) { acc[m] = 0.f; cmp[m] = 0.f; }
@@ -200,23 +205,21 @@ __device__ __forceinline__ void batch_march(const ItemDesc& it, const ItemTex<M>
 
 
 
-// One ray.  ADJOINT: the fused forward + loss + adjoint; returns the ray's
-// loss term.
+// One ray (of a lane with on set; the whole warp calls it).  ADJOINT: the
+// fused forward + loss + adjoint; returns the ray's loss term.
 template <int M, int MODE, bool ADJOINT, bool AXIS>
-__device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M>& tx, const float* s_mu, int p, int v,
-                                             int u)
+__device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M>& tx, const float* s_mu, bool on, int set,
+                                             int p, int v, int u)
 {
+    if (!ADJOINT && !on) return 0.f;
     const int64_t npix = (int64_t)it.g.U * it.g.V;
     const int64_t pix = (int64_t)v * it.g.U + u;
     const int64_t ray = (int64_t)p * npix + pix;
-    const RaySeg s = ray_segment(it.g, p, v, u);
-    RayRef32 r;
-    if (MODE != INTERP_TRILINEAR) r = ray_ref32(it.g, p, v, u);
     float L[M];
-    batch_march<M, MODE, AXIS>(it, tx, s, r, p, v, u, L);
     // the plain forward's epilogue (spectral / spectral_adjoint), so the
     // batch's I equals ctfp_forward's for the same path integrals
     if (!ADJOINT) {
+        batch_march<M, MODE, AXIS>(it, tx, p, v, u, L);
         float I, A;
         spectral<M>(s_mu, it.E, it.W, pix, npix, L, I, A);
         if (it.I) it.I[ray] = I;
@@ -227,25 +230,31 @@ __device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M
         }
         return 0.f;
     }
-    float I, S[M];
-    spectral_adjoint<M>(s_mu, it.E, it.W, pix, npix, L, I, S);
-    if (it.I) it.I[ray] = I;
-    // loss (log I - log T)^2: dLoss/dI = 2 (log I - log T) / I, dI/dL_m = -S_m
-    if (!(I > 0.f)) return 0.f;
-    const float res = logf(I) - logf(it.I_target[ray]);
-    const float gI = 2.0f * res / I;
-    float g[M];
+    float g[M], res = 0.f;
     bool any = false;
 #pragma unroll
-    for (int m = 0; m < M; m++) {
-        g[m] = -gI * S[m] * it.g.dx;
-        any |= g[m] != 0.f;
+    for (int m = 0; m < M; m++) g[m] = 0.f;
+    if (on) {
+        batch_march<M, MODE, AXIS>(it, tx, p, v, u, L);
+        float I, S[M];
+        spectral_adjoint<M>(s_mu, it.E, it.W, pix, npix, L, I, S);
+        if (it.I) it.I[ray] = I;
+        // loss (log I - log T)^2: dLoss/dI = 2 (log I - log T) / I, dI/dL_m = -S_m
+        if (I > 0.f) {
+            res = logf(I) - logf(it.I_target[ray]);
+            const float gI = 2.0f * res / I;
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                g[m] = -gI * S[m] * it.g.dx;
+                any |= g[m] != 0.f;
+            }
+        }
     }
     // TEXTURE: the transpose of the texture unit's weights, which the
     // emulation reproduces exactly (as ctfp_backward does for such a plan)
-    if (any)
-        scatter_ray_axis<M, MODE == INTERP_TRILINEAR ? INTERP_TRILINEAR : INTERP_TEXEMU>(it.g, it.gexp, p, v, u, g,
-                                                                                          axis_is_x(it.g, p));
+    constexpr int SM = MODE == INTERP_TRILINEAR ? INTERP_TRILINEAR : INTERP_TEXEMU;
+    if (!AXIS && !it.gcol) scatter_direct<M, SM>(it.g, it.gvol, any, p, v, u, g);
+    else scatter_columns<M, SM>(it.g, it.gcol + (size_t)set * it.set_floats, any, p, v, u, g);
     return res * res;
 }
 
@@ -282,7 +291,7 @@ __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJO
     // and row, and whether the item changed.  Every thread re-reads these
     // (volatile) where it needs them, so none of them is held in a register
     // across a ray's march.
-    __shared__ int s_end, s_item, s_new, s_p, s_tu, s_tv;
+    __shared__ int s_end, s_item, s_new, s_p, s_tu, s_tv, s_set;
     // the current item and its unit range (thread 0): the units a CTA takes
     // mostly fall in one item, so the item search runs only when the item
     // changes
@@ -317,6 +326,7 @@ __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJO
                     const int rem = (int)(local % band_units);
                     s_tv = (int)(local / band_units);
                     s_p = rem / it.tiles_u;
+                    s_set = s_p / it.set_groups;
                     s_tu = rem % it.tiles_u;
                 } else {
                     const int tiles = it.tiles_u * it.tiles_v;
@@ -343,7 +353,11 @@ __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJO
             // this thread's ray within the unit's tile
             const int tile_u = 1 << a.tu_shift, tile_v = kThreads >> a.tu_shift;
             int du, dv;
-            if (AXIS && tile_v % 4 == 0 && tile_u <= kThreads / 4) {
+            if (ADJOINT) {
+                // lanes down the detector's rows: the scatter's runs of memory
+                du = threadIdx.x / tile_v;
+                dv = threadIdx.x % tile_v;
+            } else if (AXIS && tile_v % 4 == 0 && tile_u <= kThreads / 4) {
                 // the axis sampler's lane quads run down 4 detector rows
                 const int q = threadIdx.x >> 2;
                 du = q % tile_u;
@@ -355,7 +369,8 @@ __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJO
             const int u = *(volatile int*)&s_tu * tile_u + du;
             const int v = *(volatile int*)&s_tv * tile_v + dv;
             const int pk = *(volatile int*)&s_p * (MULTI ? a.vpu : 1) + k;
-            if (u < it.g.U && v < it.g.V && pk < it.g.P) loss += process_ray<M, MODE, ADJOINT, AXIS>(it, tx, s_mu, pk, v, u);
+            if (pk >= it.g.P) break;
+            loss += process_ray<M, MODE, ADJOINT, AXIS>(it, tx, s_mu, u < it.g.U && v < it.g.V, ADJOINT ? s_set : 0, pk, v, u);
         }
         if (ADJOINT) {
             const ItemDesc& it = a.items[*(volatile int*)&s_item];
@@ -374,22 +389,27 @@ __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJO
     }
 }
 
-// Folds every item's corner-expanded accumulators into its gradients.
-__global__ void k_batch_fold(const ItemDesc* items, int n_items, const long long* vox0, long long total)
+// Folds every item's accumulators into its gradients: one block per 32 x 32
+// (x, z) tile and y of an item, tile0[k] the first block of item k.
+__global__ void __launch_bounds__(256) k_batch_fold(const ItemDesc* items, int n_items, const long long* tile0)
 {
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        int lo = 0, hi = n_items - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (vox0[mid] <= t) lo = mid;
-            else hi = mid - 1;
-        }
-        const ItemDesc& it = items[lo];
-        const long long k = t - vox0[lo];
-        const int nx = it.g.nx, ny = it.g.ny, nz = it.g.nz;
-        const int x = (int)(k % nx), y = (int)((k / nx) % ny), z = (int)(k / ((long long)nx * ny));
-        for (int m = 0; m < it.M; m++) it.gvol[m][k] += face_fold(it.gexp[m], nx, ny, nz, x, y, z);
+    __shared__ float t[kMaxM][32][33];
+    int lo = 0, hi = n_items - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tile0[mid] <= (long long)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const ItemDesc& it = items[lo];
+    const int nx = it.g.nx, ny = it.g.ny, nz = it.g.nz;
+    int x0, y, z0;
+    column_tile((unsigned)((long long)blockIdx.x - tile0[lo]), nx, nz, x0, y, z0);
+    switch (it.gcol ? it.M : 0) {
+        case 0: break;
+        case 1: fold_tile<1>(it.gcol, it.sets, it.set_floats, it.gvol, nx, ny, nz, x0, y, z0, t); break;
+        case 2: fold_tile<2>(it.gcol, it.sets, it.set_floats, it.gvol, nx, ny, nz, x0, y, z0, t); break;
+        case 3: fold_tile<3>(it.gcol, it.sets, it.set_floats, it.gvol, nx, ny, nz, x0, y, z0, t); break;
+        default: fold_tile<4>(it.gcol, it.sets, it.set_floats, it.gvol, nx, ny, nz, x0, y, z0, t); break;
     }
 }
 
@@ -439,7 +459,7 @@ struct ctfp_batch {
     std::vector<ctfp_plan*> plans;
     std::vector<int> order;            // item slot -> plan index (grouped, cost order within a group)
     std::vector<bool> item_axis;       // slot -> the plan marches the axis sampler's copies
-    std::vector<long long> vox0;       // first voxel of each slot in the fold's flat index
+    std::vector<long long> tile0;      // first block of each slot in the fold's grid
     std::vector<ItemDesc> items;       // tables of the current call
     struct Group {
         int M, interp, axis, first, count;
@@ -448,12 +468,12 @@ struct ctfp_batch {
     };
     std::vector<Group> groups;
     ItemDesc* d_items[2] = {nullptr, nullptr};  // device tables of the forward, forward + adjoint graphs
-    long long* d_vox0 = nullptr;
-    long long total_units = 0, total_vox = 0;
+    long long* d_tile0 = nullptr;
+    long long total_units = 0, total_tiles = 0;
     unsigned long long* d_counter = nullptr;    // one per group
-    float4* d_gexp = nullptr;          // all items' accumulators, contiguous
-    size_t gexp_elems = 0;
-    std::vector<size_t> gexp_off;      // [slot][m]
+    float* d_gcol = nullptr;           // all items' accumulators, contiguous
+    size_t gcol_floats = 0;
+    std::vector<size_t> gcol_off;      // [slot]
     cudaStream_t capture = nullptr;    // private stream the graphs are recorded on
     // one graph per kind, valid for the tables, volume pointers and loss
     // pointer it was recorded with; it runs in the order of the stream it is
@@ -497,7 +517,7 @@ ctfp_status record(ctfp_batch* b, bool adjoint, const std::vector<const float*>&
     BATCH_CUDA(cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long) * b->groups.size(), st));
     if (adjoint) {
         // (tuning leaves the accumulators as they are: a real call zeroes them)
-        if (tune_div == 0) BATCH_CUDA(cudaMemsetAsync(b->d_gexp, 0, b->gexp_elems * sizeof(float4), st));
+        if (tune_div == 0) BATCH_CUDA(cudaMemsetAsync(b->d_gcol, 0, b->gcol_floats * sizeof(float), st));
         if (loss) BATCH_CUDA(cudaMemsetAsync(loss, 0, sizeof(float) * (size_t)b->n, st));
     }
     const ItemDesc* table = b->d_items[adjoint ? 1 : 0];
@@ -514,9 +534,7 @@ ctfp_status record(ctfp_batch* b, bool adjoint, const std::vector<const float*>&
         BATCH_CUDA(cudaGetLastError());
     }
     if (adjoint && tune_div == 0) {
-        long long nb = (b->total_vox + 255) / 256;
-        if (nb > 148 * 16) nb = 148 * 16;
-        k_batch_fold<<<(unsigned)std::max<long long>(nb, 1), 256, 0, st>>>(table, b->n, b->d_vox0, b->total_vox);
+        k_batch_fold<<<(unsigned)b->total_tiles, dim3(32, 8), 0, st>>>(table, b->n, b->d_tile0);
         BATCH_CUDA(cudaGetLastError());
     }
     return CTFP_OK;
@@ -636,11 +654,14 @@ ctfp_status fill_items(ctfp_batch* b, int kind)
             it.xtex[m] = plan_xtex(p, m);
             it.ytex[m] = plan_ytex(p, m);
             it.tex[m] = plan_tex(p, m);
-            it.gexp[m] = b->d_gexp + b->gexp_off[(size_t)s * kMaxM + m];
         }
+        it.gcol = column_fits(it.g.nx, it.g.ny, it.g.nz) ? b->d_gcol + b->gcol_off[(size_t)s] : nullptr;
         it.tiles_u = (it.g.U + b->tile_u[kind] - 1) / b->tile_u[kind];
         it.tiles_v = (it.g.V + b->tile_v[kind] - 1) / b->tile_v[kind];
         it.vgroups = (it.g.P + b->vpu[kind] - 1) / b->vpu[kind];
+        it.set_floats = accum_floats(it.g.nx, it.g.ny, it.g.nz, it.M);
+        it.set_groups = (it.vgroups + accum_sets(it.g, it.g.P, it.M) - 1) / accum_sets(it.g, it.g.P, it.M);
+        it.sets = (it.vgroups + it.set_groups - 1) / it.set_groups;
         it.unit0 = unit0;
         it.units = units;
     }
@@ -694,10 +715,10 @@ ctfp_status ctfp_batch_create(int32_t n_items, ctfp_plan* const* plans, ctfp_bat
     });
     b->items.resize((size_t)n_items);
     b->item_axis.resize((size_t)n_items);
-    b->vox0.resize((size_t)n_items);
-    b->gexp_off.assign((size_t)n_items * kMaxM, 0);
-    long long unit = 0, vox = 0;
-    size_t gexp = 0;
+    b->tile0.resize((size_t)n_items);
+    b->gcol_off.assign((size_t)n_items, 0);
+    long long unit = 0, tiles = 0;
+    size_t gcol = 0;
     for (int s = 0; s < n_items; s++) {
         ctfp_plan* p = plans[b->order[(size_t)s]];
         const GeomParams& g = plan_geom(p);
@@ -710,23 +731,21 @@ ctfp_status ctfp_batch_create(int32_t n_items, ctfp_plan* const* plans, ctfp_bat
             b->groups.back().axis != ax)
             b->groups.push_back({it.M, it.interp, ax, s, 0, unit, unit, {0, 0}});
         b->groups.back().count++;
-        b->vox0[(size_t)s] = vox;
-        vox += (long long)g.nx * g.ny * g.nz;
-        for (int m = 0; m < it.M; m++) {
-            b->gexp_off[(size_t)s * kMaxM + m] = gexp;
-            gexp += expanded_elems(g);
-        }
+        b->tile0[(size_t)s] = tiles;
+        tiles += column_tiles(g.nx, g.ny, g.nz);
+        b->gcol_off[(size_t)s] = gcol;
+        if (column_fits(g.nx, g.ny, g.nz)) gcol += (accum_floats(g.nx, g.ny, g.nz, it.M) * accum_sets(g, g.P, it.M) + 63) / 64 * 64;  // each item's on a 256-byte boundary
     }
     layout_units(b, 0);
-    b->total_vox = vox;
-    b->gexp_elems = gexp;
+    b->total_tiles = tiles;
+    b->gcol_floats = gcol;
     cudaError_t e = cudaMalloc(&b->d_items[0], sizeof(ItemDesc) * (size_t)n_items);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_items[1], sizeof(ItemDesc) * (size_t)n_items);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_vox0, sizeof(long long) * (size_t)n_items);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_tile0, sizeof(long long) * (size_t)n_items);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, sizeof(unsigned long long) * b->groups.size());
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_gexp, sizeof(float4) * gexp);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_gcol, sizeof(float) * std::max<size_t>(gcol, 1));
     if (e == cudaSuccess)
-        e = cudaMemcpy(b->d_vox0, b->vox0.data(), sizeof(long long) * (size_t)n_items, cudaMemcpyHostToDevice);
+        e = cudaMemcpy(b->d_tile0, b->tile0.data(), sizeof(long long) * (size_t)n_items, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);
     int nsm = 0;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -760,9 +779,9 @@ ctfp_status ctfp_batch_destroy(ctfp_batch* b)
         if (b->graph[i].exec) cudaGraphExecDestroy(b->graph[i].exec);
     cudaFree(b->d_items[0]);
     cudaFree(b->d_items[1]);
-    cudaFree(b->d_vox0);
+    cudaFree(b->d_tile0);
     cudaFree(b->d_counter);
-    cudaFree(b->d_gexp);
+    cudaFree(b->d_gcol);
     if (b->capture) cudaStreamDestroy(b->capture);
     delete b;
     return CTFP_OK;

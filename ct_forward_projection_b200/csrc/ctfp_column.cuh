@@ -1,0 +1,410 @@
+// ctfp_column.cuh — the adjoint's scatter (SAMPLER_AXIS's march transposed)
+// into z-fastest accumulators, shared by the plan kernel (k_backward) and the
+// batched persistent kernels.
+#pragma once
+
+#include <cmath>
+
+#include "ctfp_axis.cuh"
+#include "ctfp_device.cuh"
+
+namespace ctfp {
+
+// The accumulators: voxel (x, y, z) is element ((x + 2) * ny' + (y + 2)) * nz' +
+// (z + 2), ny' = ny + 4, nz' = nz + 4.  Two border voxels surround the volume on
+// every side, so a footprint with its base in [-2, n] on each axis lies in
+// bounds with no test; what falls into the border is never read.  One set
+// serves the views marched along x and those marched along y, and with lanes
+// down the detector's rows (z) a warp's reductions are runs of memory.
+constexpr int kColPad = 2;
+struct ColumnDims {
+    unsigned sx, sy, origin;  // element strides of x and y; element of voxel (0, 0, 0)
+    size_t elems;
+};
+__host__ __device__ __forceinline__ ColumnDims column_dims(int nx, int ny, int nz)
+{
+    ColumnDims d;
+    d.sy = (unsigned)(nz + 2 * kColPad);
+    d.sx = d.sy * (unsigned)(ny + 2 * kColPad);
+    d.origin = kColPad * (d.sx + d.sy + 1u);
+    d.elems = (size_t)d.sx * (size_t)(nx + 2 * kColPad);
+    return d;
+}
+// Whether 32-bit elements reach the whole set (a volume of over 1.4e9 voxels
+// with an extent below 5 may not fit; every other one does).
+__host__ __device__ __forceinline__ bool column_fits(int nx, int ny, int nz)
+{
+    return (double)(nx + 2 * kColPad) * (ny + 2 * kColPad) * (nz + 2 * kColPad) < 4294967040.0;
+}
+// 32 x 32 (x, z) tiles of every y: how the gradients are folded; block k's tile.
+__host__ __device__ __forceinline__ long long column_tiles(int nx, int ny, int nz)
+{
+    return (long long)((nx + 31) / 32) * ((nz + 31) / 32) * ny;
+}
+__device__ __forceinline__ void column_tile(unsigned k, int nx, int nz, int& x0, int& y, int& z0)
+{
+    const unsigned bx = (unsigned)(nx + 31) / 32, bz = (unsigned)(nz + 31) / 32;
+    x0 = (int)(k % bx) * 32;
+    z0 = (int)((k / bx) % bz) * 32;
+    y = (int)(k / (bx * bz));
+}
+// Clip of one axis to lo < a + b i < hi in samples, r = 1 / b: the first and
+// last sample are exact up to 1e-6 of a sample (outwards), so a footprint at
+// either end overhangs the volume by its border only.
+__device__ __forceinline__ void clip_tight(double a, double b, double lo, double hi, int& i0, int& i1)
+{
+    if (fabs(b) < 1e-12) {
+        if (!(a > lo && a < hi)) i1 = i0;
+        return;
+    }
+    const double r = 1.0 / b;
+    const double t0 = (lo - a) * r, t1 = (hi - a) * r;
+    const double f0 = ceil(fmin(t0, t1) - 1e-6), f1 = floor(fmax(t0, t1) + 1e-6) + 1.0;
+    if (f0 > (double)i0) i0 = (f0 > 2e9) ? 2000000000 : (int)f0;
+    if (f1 < (double)i1) i1 = (f1 < -2e9) ? -2000000000 : (int)f1;
+}
+
+// ray_segment's coordinates with one reciprocal of R and the plan's
+// reciprocals of the voxel sizes (each within 2^-52 relative of the quotient:
+// 1e-13 voxel), clipped by clip_tight to (-1 - slack, n + slack).
+__device__ __forceinline__ RaySeg column_segment(const GeomParams& g, int p, int v, int u, double slack)
+{
+    const double dsz = g.dSize, sdd = g.sdd, sod = g.sod;
+    const double detU = (double)g.dHalfLU - dsz / 2 - (double)u * dsz;
+    const double detV = (double)g.dHalfLV - dsz / 2 - (double)v * dsz;
+    const double s2 = sdd * sdd, u2 = detU * detU, v2 = detV * detV;
+    const double rR = 1.0 / sqrt(s2 + u2 + v2);
+    const double cosG = sqrt(s2 + u2) * rR;
+    const double A = cosG * (sqrt(s2 + v2) * rR), B = cosG * (detU * rR), C = detV * rR;
+    const double t0 = sod - (double)g.FOVR + (double)g.dx / 2, dt = g.dx;
+    const double2 cs = g.trig[p];
+    const double cth = cs.x, sth = cs.y;
+    double fu = 0.0, fv = 0.0;
+    if (g.fspot) {
+        const float2 f = g.fspot[p];
+        fu = f.x;
+        fv = f.y;
+    }
+    const double ku = A * cth - B * sth, cu = -sod * cth + (double)g.pHalfX;
+    const double kv = -(A * sth + B * cth), cv = sod * sth + (double)g.pHalfY + fu;
+    const double kw = -C, cw = (double)g.pHalfZ + fv;
+    RaySeg s;
+    s.ax = (ku * t0 + cu) * g.qx; s.bx = ku * dt * g.qx;
+    s.ay = (kv * t0 + cv) * g.qy; s.by = kv * dt * g.qy;
+    s.az = (kw * t0 + cw) * g.qz; s.bz = kw * dt * g.qz;
+    s.i0 = 0;
+    s.i1 = g.K;
+    clip_tight(s.ax, s.bx, -1.0 - slack, (double)g.nx + slack, s.i0, s.i1);
+    clip_tight(s.ay, s.by, -1.0 - slack, (double)g.ny + slack, s.i0, s.i1);
+    clip_tight(s.az, s.bz, -1.0 - slack, (double)g.nz + slack, s.i0, s.i1);
+    if (s.i1 < s.i0) s.i1 = s.i0;
+    return s;
+}
+
+// ---------------------------------------------------------------------------
+// Adjoint: the transposed weights of one ray's samples into the accumulators.
+// For one and two materials an element is a pair cell, the sums of voxels z and
+// z + 1 of its column (2 M floats); for three and four it is voxel z (4 floats).
+// Either way a face of 2 x 2 voxels is two columns, and a column one reduction
+// of at most 16 bytes (pair cells) or two.
+//
+// What binds the scatter is the L2's rate of reduced sectors (a probe: 1.9e11
+// scattered reductions of 4 to 16 bytes a second, 3.5e11 of 16 bytes in runs of
+// 8 lanes or more, 1.4e12 floats a second at most) and, once the accumulators
+// outgrow the L2, DRAM.  Hence z-fastest elements with lanes down the rows
+// (runs), no copy of a voxel per face corner or march axis (2 or 1.3 floats per
+// voxel and material instead of 8), pair cells where an element would be less
+// than half a sector, and for 16-byte elements the hand-over in flush_voxels.
+// Against the face-expanded layout this replaced (adjoint + fold): 256^3, 90
+// views, 2 materials 18.4 -> 14.0 ms; 3 materials 34.3 -> 17.0 ms; 128^3, 60
+// views, 1 material 3.2 -> 2.4 ms; 512^3, 48 views, 4 materials 558 -> 260 ms.
+__host__ __device__ constexpr int accum_width(int M) { return M <= 2 ? 2 * M : 4; }
+
+// Sets of accumulators an adjoint over n views sums into (contiguous ranges of
+// the views, folded together): an FP32 sum of many small terms loses about
+// sqrt(terms) ulp of itself, and K sets of a K-th of the terms lose a K-th of
+// that.  At most as many as keep the gradients' error against FP64 at that of
+// separate accumulators per face corner and march axis (8 per voxel); fewer
+// where a voxel collects few rays (n views of one ray per voxel face each).
+// 2-norm relative error, one set / these sets / those 8: 97 x 113 x 75 voxels, 2
+// materials, 41 views 1.5e-7 / 6.4e-8 / 5.8e-8; 256^3, 3 materials, 90 views
+// 2.5e-7 / 1.1e-7 / 1.0e-7; 360 views, 2 materials (4 sets) 1.3e-7 against 1.2e-7.
+inline int accum_sets(const GeomParams& g, int n, int M)
+{
+    const float pitch = g.dSize * g.sod / g.sdd;
+    const float rays = (float)n * g.pSizeZ * fminf(g.pSizeX, g.pSizeY) / (pitch * pitch);
+    const int most = M <= 2 ? 4 : 6, k = rays < 6.f * most ? (int)ceilf(rays / 6.f) : most;
+    return k < 1 ? 1 : (k < n ? k : n);
+}
+
+__device__ __forceinline__ void red_v2(float* q, float a, float b)
+{
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(q), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void red_v4(float* q, float a, float b, float c, float d)
+{
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(q), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void red_v4_if(bool on, float* q, float a, float b, float c, float d)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t"
+                 "@p red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" ::"l"(q), "f"(a), "f"(b), "f"(c), "f"(d),
+                 "r"((unsigned)on)
+                 : "memory");
+}
+
+// One ray's face sums on their way into memory: slot 0 the even layer, slot 1
+// the odd one of its current pair, each the summed weights of (a, b),
+// (a + 1, b), (a, b + 1), (a + 1, b + 1); a slot is flushed when its layer or
+// the in-layer base changes.  Above two materials the whole warp calls move()
+// and finish() together.
+template <int M>
+struct ColumnScatter {
+    static constexpr bool warp_wide = M > 2;
+    float* acc;
+    const float* g;  // dLoss/dL_m times dx
+    unsigned sA;
+    unsigned h0, h1;  // element of the slot's face, kNone before the first sample
+    float s0[4], s1[4];
+    static constexpr unsigned kNone = 0xffffffffu;
+
+    __device__ __forceinline__ void begin(float* a, const float* gg, unsigned sa)
+    {
+        acc = a;
+        g = gg;
+        sA = sa;
+        h0 = h1 = kNone;
+#pragma unroll
+        for (int j = 0; j < 4; j++) s0[j] = s1[j] = 0.f;
+    }
+
+    // Pair cells, one lane on its own.
+    __device__ __forceinline__ void flush_cells(unsigned at, const float* s) const
+    {
+        constexpr int W = accum_width(M);
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            float* q = acc + (size_t)(at + (c ? sA : 0u)) * W;
+            if (M == 1) red_v2(q, s[c] * g[0], s[c + 2] * g[0]);
+            else red_v4(q, s[c] * g[0], s[c] * g[M - 1], s[c + 2] * g[0], s[c + 2] * g[M - 1]);
+        }
+    }
+
+    // Single voxels, the lanes with need set.  Lanes run down the detector's
+    // rows, about one voxel apart in z, so a lane's upper voxel is mostly the
+    // next lane's lower one: where both flush the same column together, the
+    // lane hands its upper sums over and one reduction covers both.
+    __device__ __forceinline__ void flush_voxels(bool need, unsigned at, const float* s) const
+    {
+        constexpr unsigned full = 0xffffffffu;
+        const unsigned key = need ? at : kNone;
+        const unsigned below = __shfl_up_sync(full, key, 1);
+        const bool take = need && below + 1u == key;
+        const unsigned takers = __ballot_sync(full, take);  // (every lane: not in a short-circuited operand)
+        const bool alone = need && !(takers >> 1 >> (threadIdx.x & 31u) & 1u);
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            float* q = acc + (size_t)((need ? at : 0u) + (c ? sA : 0u)) * 4;
+            float lo[4], hi[4];
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                lo[m] = hi[m] = 0.f;
+                if (m < M) {
+                    hi[m] = s[c + 2] * g[m < M ? m : 0];
+                    const float r = __shfl_up_sync(full, hi[m], 1);
+                    lo[m] = fmaf(s[c], g[m < M ? m : 0], take ? r : 0.f);
+                }
+            }
+            red_v4_if(need, q, lo[0], lo[1], lo[2], lo[3]);
+            red_v4_if(alone, q + 4, hi[0], hi[1], hi[2], hi[3]);
+        }
+    }
+
+    __device__ __forceinline__ void flush(bool need, unsigned at, const float* s) const
+    {
+        if (M > 2) flush_voxels(need, at, s);
+        else if (need) flush_cells(at, s);
+    }
+
+    __device__ __forceinline__ void slot(bool live, unsigned f, unsigned& h, float* s)
+    {
+        const bool change = live && f != h;
+        if (warp_wide ? __any_sync(0xffffffffu, change) : change) {
+            flush(change && h != kNone, h, s);
+#pragma unroll
+            for (int j = 0; j < 4; j++) s[j] = change ? 0.f : s[j];
+            if (change) h = f;
+        }
+    }
+    __device__ __forceinline__ void move(bool live, unsigned f0, unsigned f1)
+    {
+        slot(live, f0, h0, s0);
+        slot(live, f1, h1, s1);
+    }
+    __device__ __forceinline__ void finish() const
+    {
+        flush(h0 != kNone, h0, s0);
+        flush(h1 != kNone, h1, s1);
+    }
+    // The samples a ray of n steps through: those of the warp's longest ray
+    // when the warp flushes together.
+    static __device__ __forceinline__ int steps(int n)
+    {
+        return warp_wide ? __reduce_max_sync(0xffffffffu, n) : n;
+    }
+};
+
+template <int M>
+__device__ __forceinline__ void scatter_trilinear(const GeomParams& gp, float* acc, bool on, int p, int v, int u,
+                                                  const float* g)
+{
+    RaySeg s = column_segment(gp, p, v, u, 0.0);
+    const ColumnDims cd = column_dims(gp.nx, gp.ny, gp.nz);
+    const bool xl = axis_is_x(gp, p);
+    const double bl = xl ? s.bx : s.by, ba = xl ? s.by : s.bx, bz = s.bz;
+    const double i0 = (double)s.i0;
+    double cl = fma(i0, bl, xl ? s.ax : s.ay), ca = fma(i0, ba, xl ? s.ay : s.ax), cz = fma(i0, bz, s.az);
+    const unsigned sL = xl ? cd.sx : cd.sy, sA = xl ? cd.sy : cd.sx;
+    using Scatter = ColumnScatter<M>;
+    const int n = on ? s.i1 - s.i0 : 0, steps = Scatter::steps(n);
+    Scatter k;
+    k.begin(acc, g, sA);
+#pragma unroll(Scatter::warp_wide ? 1 : 2)
+    for (int i = 0; i < steps; i++) {
+        float wl, ul, wa, ua, wz, uz;
+        const int il = axis_weights(cl, wl, ul), ia = axis_weights(ca, wa, ua), iz = axis_weights(cz, wz, uz);
+        cl += bl;
+        ca += ba;
+        cz += bz;
+        const unsigned lo = (unsigned)il * sL + ((unsigned)ia * sA + (unsigned)(iz + (int)cd.origin)), hi = lo + sL;
+        const bool par = il & 1, live = !Scatter::warp_wide || i < n;
+        k.move(live, par ? hi : lo, par ? lo : hi);
+        if (!live) continue;
+        const float w0 = par ? wl : ul, w1 = par ? ul : wl;
+        const float w[4] = {ua * uz, wa * uz, ua * wz, wa * wz};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            k.s0[j] = fmaf(w[j], w0, k.s0[j]);
+            k.s1[j] = fmaf(w[j], w1, k.s1[j]);
+        }
+    }
+    k.finish();
+}
+
+template <int M, bool XL>
+__device__ __forceinline__ void scatter_texemu(const GeomParams& gp, float* acc, bool on, int p, int v, int u,
+                                               const float* g)
+{
+    const RaySeg s = column_segment(gp, p, v, u, 0.5);
+    const RayRef32 r = ray_ref32(gp, p, v, u);
+    const ColumnDims cd = column_dims(gp.nx, gp.ny, gp.nz);
+    const unsigned sL = XL ? cd.sx : cd.sy, sA = XL ? cd.sy : cd.sx;
+    using Scatter = ColumnScatter<M>;
+    const int n = on ? s.i1 - s.i0 : 0, steps = Scatter::steps(n);
+    Scatter k;
+    k.begin(acc, g, sA);
+    for (int i = 0; i < steps; i++) {
+        const Corner c = corner_tex(ref32_coords(gp, r, s.i0 + i));
+        const int x = __vimin_s32_relu(c.ix + kColPad, gp.nx + kColPad);
+        const int y = __vimin_s32_relu(c.iy + kColPad, gp.ny + kColPad);
+        const int z = __vimin_s32_relu(c.iz + kColPad, gp.nz + kColPad);
+        const unsigned lo = (unsigned)x * cd.sx + (unsigned)y * cd.sy + (unsigned)z, hi = lo + sL;
+        const bool par = (XL ? x : y) & 1, live = !Scatter::warp_wide || i < n;
+        k.move(live, par ? hi : lo, par ? lo : hi);
+        if (!live) continue;
+        float w[8];
+        texunit_weights(c.qx, c.qy, c.qz, w);
+        constexpr int lb = XL ? 1 : 2, ab = XL ? 2 : 1;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int q = (j & 2 ? 4 : 0) + (j & 1 ? ab : 0);
+            k.s0[j] += par ? w[q + lb] : w[q];
+            k.s1[j] += par ? w[q] : w[q + lb];
+        }
+    }
+    k.finish();
+}
+
+// The adjoint of one ray's march, scaled by g[m] = dLoss/dL_m times dx, for
+// the lanes with on set; every lane of the warp calls it, for the same view.
+template <int M, int MODE>
+__device__ __forceinline__ void scatter_columns(const GeomParams& gp, float* acc, bool on, int p, int v, int u,
+                                                const float* g)
+{
+    if (!ColumnScatter<M>::warp_wide && !on) return;
+    if (MODE == INTERP_TRILINEAR) scatter_trilinear<M>(gp, acc, on, p, v, u, g);
+    else if (axis_is_x(gp, p)) scatter_texemu<M, true>(gp, acc, on, p, v, u, g);
+    else scatter_texemu<M, false>(gp, acc, on, p, v, u, g);
+}
+
+// The same for a volume that column_fits refuses: every voxel of every sample
+// by an atomic addition into the gradients.
+template <int M, int MODE>
+__device__ __noinline__ void scatter_direct(const GeomParams& gp, float* const* gvol, bool on, int p, int v, int u,
+                                            const float* g)
+{
+    if (!on) return;
+    const RaySeg s = ray_segment(gp, p, v, u);
+    const RayRef32 r = ray_ref32(gp, p, v, u);
+    for (int i = s.i0; i < s.i1; i++) {
+        const double t = (double)i;
+        const Corner c = MODE == INTERP_TRILINEAR
+                             ? corner_of<INTERP_TRILINEAR>(fma(t, s.bx, s.ax), fma(t, s.by, s.ay), fma(t, s.bz, s.az))
+                             : corner_tex(ref32_coords(gp, r, i));
+        float w[8];
+        corner_weights<MODE>(c, w);
+        for (int k = 0; k < 8; k++) {
+            const int x = c.ix + (k & 1), y = c.iy + (k >> 1 & 1), z = c.iz + (k >> 2);
+            if ((unsigned)x >= (unsigned)gp.nx || (unsigned)y >= (unsigned)gp.ny || (unsigned)z >= (unsigned)gp.nz) continue;
+            const size_t at = ((size_t)z * gp.ny + y) * gp.nx + x;
+            for (int m = 0; m < M; m++) atomicAdd(gvol[m] + at, w[k] * g[m]);
+        }
+    }
+}
+
+// Adds `sets` sets of accumulators, stride floats apart, of a 32 x 32 (x, z)
+// tile of one y into the gradients: read along z, turned in shared memory
+// t[M][32][33], written along x.  The block is 32 x 8 threads.
+template <int M>
+__device__ __forceinline__ void fold_tile(const float* __restrict__ acc, int sets, size_t stride, float* const* g, int nx,
+                                          int ny, int nz, int x0, int y, int z0, float (*t)[32][33])
+{
+    const ColumnDims cd = column_dims(nx, ny, nz);
+    const int tx = threadIdx.x;
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int x = x0 + k, z = z0 + tx;
+        if (x < nx && z < nz) {
+            const float* q =
+                acc + ((size_t)x * cd.sx + (size_t)y * cd.sy + (size_t)z + cd.origin) * accum_width(M);
+            // pair cells: voxel z is the first half of cell z and the second of cell z - 1
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int j = 0; j < sets; j++, q += stride) {
+                if (M == 1) {
+                    v[0] += q[0] + q[-1];
+                } else if (M == 2) {
+                    const float2 e = *(const float2*)q, f = *(const float2*)(q - 2);
+                    v[0] += e.x + f.x;
+                    v[1] += e.y + f.y;
+                } else {
+                    const float4 e = *(const float4*)q;
+                    v[0] += e.x;
+                    v[1] += e.y;
+                    v[2] += e.z;
+                    v[3] += e.w;
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < M; m++) t[m][tx][k] = v[m];
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int x = x0 + tx, z = z0 + k;
+        if (x < nx && z < nz) {
+#pragma unroll
+            for (int m = 0; m < M; m++) g[m][((size_t)z * ny + y) * nx + x] += t[m][k][tx];
+        }
+    }
+}
+
+}  // namespace ctfp

@@ -32,6 +32,7 @@ struct GeomParams {
     float dHalfLU, dHalfLV, dSize, sod, sdd, FOVR, dx;
     float pHalfX, pHalfY, pHalfZ, pSizeX, pSizeY, pSizeZ;
     float rpSizeX, rpSizeY, rpSizeZ;  // 1 / pSize rounded to FP32 (div_rn_recip)
+    double qx, qy, qz;                // 1 / pSize in FP64 (column_segment)
     const double2* trig;     // per view (cos, sin) of the FP32 view angle
     const float2* trigf;     // the same, rounded to FP32 (compat samplers)
     const float2* fspot;     // per view focal-spot offset (u, v) in mm, or null
@@ -441,14 +442,6 @@ __device__ __forceinline__ void gather4_interp(const cudaTextureObject_t* ltex, 
 #pragma unroll
     for (int m = 0; m < M; m++) out[m] = interp8<MODE>(c, v[m]);
 }
-
-// One 16-byte vector reduction into global memory (the adjoint's accumulators).
-__device__ __forceinline__ void red_add_v4(float4* p, float a, float b, float c, float d)
-{
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
-                 : "memory");
-}
-
 
 // exp(-a) and 1 - exp(-a), each to a few ulp relative.  For |a| < 1/4 the
 // absorbed fraction is the Taylor series 1 - exp(-a) = a (1 - a/2 + a^2/6 -

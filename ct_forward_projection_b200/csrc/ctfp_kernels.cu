@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "ctfp_axis.cuh"
+#include "ctfp_column.cuh"
 #include "ctfp_kernels.cuh"
 
 namespace ctfp {
@@ -280,77 +281,84 @@ __global__ void __launch_bounds__(256) k_spectral_from_L(const MarchParams prm)
 // reductions.  FROM_GL: the input is dLoss/dL directly (transpose of the line
 // integrals).
 //
-// Grid: x = pixel tiles along u, y = view groups, z = pixel tiles along v, so
-// that the CTAs resident at any time cover one band of detector rows for many
-// views.  The rays of a row band cross a thin z-slab of the volume (the cone
+// Grid: x = pixel tiles along u, y = the view groups of a set of accumulators,
+// z = pixel tiles along v of every set, so that the CTAs resident at any time
+// cover one band of detector rows for many views.  The rays of a row band cross a thin z-slab of the volume (the cone
 // angle is small), so the accumulator cells they reduce into stay in L2; with
 // views outermost every view would sweep the whole accumulator through DRAM.
-// Register cap for 4 CTAs of 256 threads (64 registers, ~40 B of spills): the
-// poly_grid_256 adjoint 0.8 ms faster than at 3 CTAs (76 registers, none).
-template <int M, int MODE, bool FROM_GL>
-__global__ void __launch_bounds__(256, 4) k_backward(const MarchParams prm)
+// Register cap for 4 CTAs of 256 threads (64 registers): more warps hide the
+// reductions' latency.
+// DIRECT: no accumulators (prm.gcol null), the gradients take the sums.
+template <int M, int MODE, bool FROM_GL, bool DIRECT>
+__global__ void __launch_bounds__(256, 4)
+    k_backward(const MarchParams prm, int tile_u, int warp_rows, int tiles_v, int set_groups)
 {
     extern __shared__ float s_mu[];
     if (!FROM_GL) load_mu(s_mu, prm.mu, prm.E * M);
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    const int v = blockIdx.z * blockDim.y + threadIdx.y;
-    if (u >= prm.g.U || v >= prm.g.V) return;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int tile_v = (int)blockDim.x / tile_u;
+    const int wcols = 32 / warp_rows, warps_u = tile_u / wcols;
+    const int u = blockIdx.x * tile_u + (w % warps_u) * wcols + lane / warp_rows;
+    const int set = blockIdx.z / tiles_v, band = blockIdx.z % tiles_v;
+    const int v = band * tile_v + (w / warps_u) * warp_rows + lane % warp_rows;
+    const bool ray_on = u < prm.g.U && v < prm.g.V;
     const int64_t npix = (int64_t)prm.g.U * prm.g.V;
     const int64_t pix = (int64_t)v * prm.g.U + u;
     const int pend = prm.view0 + prm.n_views;
     for (int k = 0; k < prm.views_per_cta; k++) {
-        const int p = prm.view0 + blockIdx.y * prm.views_per_cta + k;
+        const int p = prm.view0 + (set * set_groups + blockIdx.y) * prm.views_per_cta + k;
         if (p >= pend) break;
         const int64_t ray = (int64_t)(p - prm.out_view0) * npix + pix;
         float g[M];
-        if (FROM_GL) {
-            load_L<M>(prm.Lin, ray, g);
-#pragma unroll
-            for (int m = 0; m < M; m++) g[m] *= prm.g.dx;
-        } else {
-            float L[M], S[M];
-            load_L<M>(prm.Lin, ray, L);
-#pragma unroll
-            for (int m = 0; m < M; m++) S[m] = 0.f;
-            // the spectral weights as the forward formed them (transmit, the
-            // same order), so S matches the fused kernels' exactly
-            for (int e = 0; e < prm.E; e++) {
-                float att = 0.f;
-#pragma unroll
-                for (int m = 0; m < M; m++) att = fmaf(s_mu[e * M + m], L[m], att);
-                float ex, om;
-                transmit(att, ex, om);
-                const float Ie = __ldg(prm.W + (int64_t)e * npix + pix) * ex;
-#pragma unroll
-                for (int m = 0; m < M; m++) S[m] = fmaf(s_mu[e * M + m], Ie, S[m]);
-            }
-            const float gd = ((prm.gIAbs ? prm.gIAbs[ray] : 0.f) - (prm.gI ? prm.gI[ray] : 0.f)) * prm.g.dx;
-#pragma unroll
-            for (int m = 0; m < M; m++) g[m] = gd * S[m];
-        }
         bool any = false;
 #pragma unroll
-        for (int m = 0; m < M; m++) any |= (g[m] != 0.f);
-        if (!any) continue;
+        for (int m = 0; m < M; m++) g[m] = 0.f;
+        if (ray_on) {
+            if (FROM_GL) {
+                load_L<M>(prm.Lin, ray, g);
+#pragma unroll
+                for (int m = 0; m < M; m++) g[m] *= prm.g.dx;
+            } else {
+                float L[M], S[M];
+                load_L<M>(prm.Lin, ray, L);
+#pragma unroll
+                for (int m = 0; m < M; m++) S[m] = 0.f;
+                // the spectral weights as the forward formed them (transmit, the
+                // same order), so S matches the fused kernels' exactly
+                for (int e = 0; e < prm.E; e++) {
+                    float att = 0.f;
+#pragma unroll
+                    for (int m = 0; m < M; m++) att = fmaf(s_mu[e * M + m], L[m], att);
+                    float ex, om;
+                    transmit(att, ex, om);
+                    const float Ie = __ldg(prm.W + (int64_t)e * npix + pix) * ex;
+#pragma unroll
+                    for (int m = 0; m < M; m++) S[m] = fmaf(s_mu[e * M + m], Ie, S[m]);
+                }
+                const float gd = ((prm.gIAbs ? prm.gIAbs[ray] : 0.f) - (prm.gI ? prm.gI[ray] : 0.f)) * prm.g.dx;
+#pragma unroll
+                for (int m = 0; m < M; m++) g[m] = gd * S[m];
+            }
+#pragma unroll
+            for (int m = 0; m < M; m++) any |= (g[m] != 0.f);
+        }
         // the transposed weights of the forward's sampler (for the texture
         // modes, the texture unit's, at the reference's FP32 coordinates)
-        scatter_ray_axis<M, MODE == INTERP_TRILINEAR ? INTERP_TRILINEAR : INTERP_TEXEMU>(
-            prm.g, prm.gexp, p, v, u, g, axis_is_x(prm.g, p));
+        constexpr int SM = MODE == INTERP_TRILINEAR ? INTERP_TRILINEAR : INTERP_TEXEMU;
+        if (DIRECT) scatter_direct<M, SM>(prm.g, prm.gvol, any, p, v, u, g);
+        else scatter_columns<M, SM>(prm.g, prm.gcol + (size_t)set * prm.set_floats, any, p, v, u, g);
     }
 }
 
-// Sums the face accumulators of both march axes into the gradient volumes
-// (face_fold).  One streaming pass.
+// Adds the accumulators into the gradient volumes (fold_tile).  Block (32, 8);
+// one block per tile, column_tile.
 template <int M>
-__global__ void k_fold(const MarchParams prm)
+__global__ void __launch_bounds__(256) k_fold(const MarchParams prm)
 {
-    const int nx = prm.g.nx, ny = prm.g.ny, nz = prm.g.nz;
-    const int64_t n = (int64_t)nx * ny * nz;
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(k % nx), y = (int)((k / nx) % ny), z = (int)(k / ((int64_t)nx * ny));
-#pragma unroll
-        for (int m = 0; m < M; m++) prm.gvol[m][k] += face_fold(prm.gexp[m], nx, ny, nz, x, y, z);
-    }
+    __shared__ float t[M][32][33];
+    int x0, y, z0;
+    column_tile(blockIdx.x, prm.g.nx, prm.g.nz, x0, y, z0);
+    fold_tile<M>(prm.gcol, prm.sets, prm.set_floats, prm.gvol, prm.g.nx, prm.g.ny, prm.g.nz, x0, y, z0, t);
 }
 
 // W[e][k] = ((I0Val * S_e) * G_e) * D_e in the reference's multiplication order
@@ -955,19 +963,28 @@ cudaError_t axis_dispatch(const MarchParams& prm, int interp, bool spec, int min
     return cudaErrorInvalidValue;
 }
 
+struct BwdGrid {
+    int tile_u, rows, tiles_v, set_groups;
+    dim3 grid, block;
+    size_t smem;
+};
+
+template <int M, int MODE, bool FROM_GL>
+cudaError_t bwd_launch(const MarchParams& prm, const BwdGrid& b, cudaStream_t st)
+{
+    const size_t smem = FROM_GL ? 0 : b.smem;
+    const auto k = prm.gcol ? k_backward<M, MODE, FROM_GL, false> : k_backward<M, MODE, FROM_GL, true>;
+    k<<<b.grid, b.block, smem, st>>>(prm, b.tile_u, b.rows, b.tiles_v, b.set_groups);
+    return cudaGetLastError();
+}
+
 template <int M>
-cudaError_t bwd_dispatch(const MarchParams& prm, int interp, bool from_gL, dim3 grid, dim3 block, size_t smem,
-                         cudaStream_t st)
+cudaError_t bwd_dispatch(const MarchParams& prm, int interp, bool from_gL, const BwdGrid& b, cudaStream_t st)
 {
     const bool tri = interp == INTERP_TRILINEAR;
-    if (from_gL) {
-        if (tri) k_backward<M, INTERP_TRILINEAR, true><<<grid, block, 0, st>>>(prm);
-        else k_backward<M, INTERP_TEXEMU, true><<<grid, block, 0, st>>>(prm);
-    } else {
-        if (tri) k_backward<M, INTERP_TRILINEAR, false><<<grid, block, smem, st>>>(prm);
-        else k_backward<M, INTERP_TEXEMU, false><<<grid, block, smem, st>>>(prm);
-    }
-    return cudaGetLastError();
+    if (from_gL)
+        return tri ? bwd_launch<M, INTERP_TRILINEAR, true>(prm, b, st) : bwd_launch<M, INTERP_TEXEMU, true>(prm, b, st);
+    return tri ? bwd_launch<M, INTERP_TRILINEAR, false>(prm, b, st) : bwd_launch<M, INTERP_TEXEMU, false>(prm, b, st);
 }
 
 dim3 march_grid(const MarchParams& prm, const LaunchShape& ls)
@@ -1117,47 +1134,77 @@ cudaError_t launch_spectral_from_L(const MarchParams& prm, int M, cudaStream_t s
     return cudaGetLastError();
 }
 
+bool accum_fits(int nx, int ny, int nz) { return column_fits(nx, ny, nz); }
+
+int accum_set_count(const GeomParams& g, int n_views, int M) { return accum_sets(g, n_views, M); }
+
+size_t accum_floats(int nx, int ny, int nz, int M) { return column_dims(nx, ny, nz).elems * accum_width(M); }
+
 cudaError_t launch_backward(const MarchParams& prm_in, int M, int interp, bool from_gL, const LaunchShape& ls,
                             cudaStream_t st)
 {
-    const dim3 block(ls.tile_u, ls.tile_v);
-    const size_t smem = sizeof(float) * (size_t)prm_in.E * M;
-    // row bands outermost (grid.z), views in grid.y: at most 65535 view
-    // groups per launch
-    const int vpc = ls.views_per_cta;
-    const int max_views = 65535 * vpc;
-    for (int v0 = 0; v0 < prm_in.n_views; v0 += max_views) {
+    // Rows of the detector a warp covers (32 / rows columns).  Its lanes' z
+    // neighbours share sectors, so taller is better until the rows stop
+    // crossing layers together: 16 rows, and 32 where the rows lie close
+    // together and several lanes flush the same cell.  Measured, adjoint +
+    // fold of 24 views of 128^3, row spacing in voxels: 8 / 16 / 32 rows, ms --
+    // 1 material 0.25: 4.72 / 3.78 / 3.75, 0.6: 1.05 / 1.02 / 1.09, 1.05: 0.46 /
+    // 0.47 / 0.49; 3 materials 0.25: 11.96 / 10.07 / 9.17, 1.05: 0.86 / 0.84 / 0.88.
+    const GeomParams& g = prm_in.g;
+    int rows = g.dSize * g.sod < 0.35f * g.sdd * g.pSizeZ ? 32 : 16;
+    while (rows > 4 && rows / 2 >= g.V) rows /= 2;
+    const int threads = ls.tile_u * ls.tile_v;
+    LaunchShape bs = ls;
+    if (bs.tile_v % rows != 0 || bs.tile_u % (32 / rows) != 0) {
+        bs.tile_v = rows;
+        bs.tile_u = threads / rows;  // a multiple of 32 / rows: whole warps
+    }
+    BwdGrid b;
+    b.tile_u = bs.tile_u;
+    b.rows = rows;
+    b.tiles_v = (prm_in.g.V + bs.tile_v - 1) / bs.tile_v;
+    b.block = dim3(threads);
+    b.smem = sizeof(float) * (size_t)prm_in.E * M;
+    const unsigned tiles_u = (unsigned)((prm_in.g.U + bs.tile_u - 1) / bs.tile_u);
+    // view groups run along grid.y, at most 65535 per launch: all sets in one
+    // launch, or past that one part of a set's views after the other
+    const int vpc = ls.views_per_cta, sets = prm_in.gcol ? prm_in.sets : 1;
+    const int groups = (prm_in.n_views + vpc - 1) / vpc;
+    b.set_groups = (groups + sets - 1) / sets;
+    const bool whole = b.set_groups <= 65535;
+    const int most = whole ? groups : 65535;
+    for (int g0 = 0; g0 < groups;) {
         MarchParams prm = prm_in;
+        const int set = whole ? 0 : g0 / b.set_groups;
+        const int n = whole ? groups : std::min(std::min(most, groups - g0), (set + 1) * b.set_groups - g0);
         prm.views_per_cta = vpc;
-        prm.view0 = prm_in.view0 + v0;
-        prm.n_views = std::min(max_views, prm_in.n_views - v0);
-        const dim3 grid((prm.g.U + ls.tile_u - 1) / ls.tile_u, (prm.n_views + vpc - 1) / vpc,
-                        (prm.g.V + ls.tile_v - 1) / ls.tile_v);
-        if (grid.x == 0 || grid.y == 0 || grid.z == 0) return cudaSuccess;
+        prm.view0 = prm_in.view0 + g0 * vpc;
+        prm.n_views = std::min(n * vpc, prm_in.n_views - g0 * vpc);
+        if (prm.gcol) prm.gcol += (size_t)set * prm.set_floats;
+        b.grid = whole ? dim3(tiles_u, b.set_groups, b.tiles_v * sets) : dim3(tiles_u, n, b.tiles_v);
+        if (b.grid.x == 0 || b.grid.y == 0 || b.grid.z == 0) return cudaSuccess;
         cudaError_t e = cudaErrorInvalidValue;
         switch (M) {
-            case 1: e = bwd_dispatch<1>(prm, interp, from_gL, grid, block, smem, st); break;
-            case 2: e = bwd_dispatch<2>(prm, interp, from_gL, grid, block, smem, st); break;
-            case 3: e = bwd_dispatch<3>(prm, interp, from_gL, grid, block, smem, st); break;
-            case 4: e = bwd_dispatch<4>(prm, interp, from_gL, grid, block, smem, st); break;
+            case 1: e = bwd_dispatch<1>(prm, interp, from_gL, b, st); break;
+            case 2: e = bwd_dispatch<2>(prm, interp, from_gL, b, st); break;
+            case 3: e = bwd_dispatch<3>(prm, interp, from_gL, b, st); break;
+            case 4: e = bwd_dispatch<4>(prm, interp, from_gL, b, st); break;
         }
         if (e != cudaSuccess) return e;
+        g0 += n;
     }
     return cudaSuccess;
 }
 
-size_t expanded_elems(const GeomParams& g) { return face_elems(g.nx, g.ny, g.nz); }
-
 cudaError_t launch_fold(const MarchParams& prm, int M, cudaStream_t st)
 {
-    const int64_t n = (int64_t)prm.g.nx * prm.g.ny * prm.g.nz;
-    int64_t nb = (n + 255) / 256;
-    if (nb > 148 * 16) nb = 148 * 16;
+    if (!prm.gcol) return cudaSuccess;
+    const dim3 grid((unsigned)column_tiles(prm.g.nx, prm.g.ny, prm.g.nz)), block(32, 8);
     switch (M) {
-        case 1: k_fold<1><<<(unsigned)nb, 256, 0, st>>>(prm); break;
-        case 2: k_fold<2><<<(unsigned)nb, 256, 0, st>>>(prm); break;
-        case 3: k_fold<3><<<(unsigned)nb, 256, 0, st>>>(prm); break;
-        case 4: k_fold<4><<<(unsigned)nb, 256, 0, st>>>(prm); break;
+        case 1: k_fold<1><<<grid, block, 0, st>>>(prm); break;
+        case 2: k_fold<2><<<grid, block, 0, st>>>(prm); break;
+        case 3: k_fold<3><<<grid, block, 0, st>>>(prm); break;
+        case 4: k_fold<4><<<grid, block, 0, st>>>(prm); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

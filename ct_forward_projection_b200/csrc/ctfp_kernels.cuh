@@ -22,7 +22,9 @@ struct MarchParams {
     const float* gI;                  // [P][V][U] dLoss/dI (adjoint)
     const float* gIAbs;               // [P][V][U] dLoss/dIAbsorb (adjoint, may be null)
     float* gvol[kMaxM];               // gradient volumes (adjoint)
-    float4* gexp[kMaxM];              // face-expanded gradient accumulators (adjoint), see AxisScatter
+    float* gcol;                      // gradient accumulators of every material (adjoint, ctfp_column.cuh)
+    int sets;                         // sets of them, set_floats apart, the views in as many contiguous parts
+    size_t set_floats;
     int E;
     int view0;                        // first view of this launch
     int n_views;                      // views in this launch
@@ -59,13 +61,15 @@ struct LaunchShape {
 cudaError_t launch_forward(const MarchParams& prm, int M, int interp, int sampler, bool do_spectral,
                            const LaunchShape& ls, cudaStream_t st);
 cudaError_t launch_spectral_from_L(const MarchParams& prm, int M, cudaStream_t st);
-// Adjoint scatter into the face-expanded accumulators prm.gexp (zeroed by
-// the caller), followed by launch_fold into prm.gvol.
+// Floats of one set of the adjoint's accumulators (accum_width).
+size_t accum_floats(int nx, int ny, int nz, int M);
+int accum_set_count(const GeomParams& g, int n_views, int M);  // accum_sets
+bool accum_fits(int nx, int ny, int nz);  // false: launch_backward adds into prm.gvol (prm.gcol null)
+// Adjoint scatter into the accumulators prm.gcol (zeroed by the caller),
+// followed by launch_fold into prm.gvol.
 cudaError_t launch_backward(const MarchParams& prm, int M, int interp, bool from_gL, const LaunchShape& ls,
                             cudaStream_t st);
 cudaError_t launch_fold(const MarchParams& prm, int M, cudaStream_t st);
-// Elements (float4) of one material's face-expanded accumulator (face_elems).
-size_t expanded_elems(const GeomParams& g);
 cudaError_t launch_weights(const float* spectrum, const float* grid, int grid_layout, const float* det,
                            float I0Val, int E, int U, int V, float* W, float* I0, cudaStream_t st);
 cudaError_t launch_finalize(int64_t n_pix, int64_t n_views, const float* I, const float* IAbs, const float* I0,
