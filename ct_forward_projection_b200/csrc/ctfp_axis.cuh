@@ -86,13 +86,19 @@ __device__ __forceinline__ Corner axis_corner(const GeomParams& g, const RayRef3
 // does not depend on the launch shape.  (Stepping a warp's lanes through
 // common sample indices instead, from the earliest entry to the latest exit
 // among them, measured 3 % slower on poly_grid_256: the extra iterations
-// cost more than the gathers the tighter lockstep saves.)
+// cost more than the gathers the tighter lockstep saves.)  part, parts: only
+// the ray's part-th of parts equal runs of samples.
 template <int M, int MODE, int AX, bool SKIP>
 __device__ __forceinline__ void march_ray_axis(const GeomParams& g, const cudaTextureObject_t* xtex,
                                                const cudaTextureObject_t* ytex, const OccView& occ, int p, int v,
-                                               int u, float* L)
+                                               int u, float* L, int part = 0, int parts = 1)
 {
-    const RaySeg s = ray_segment(g, p, v, u);
+    RaySeg s = ray_segment(g, p, v, u);
+    if (parts > 1) {
+        const int len = (s.i1 - s.i0 + parts - 1) / parts;
+        s.i0 += part * len;
+        s.i1 = min(s.i1, s.i0 + len);
+    }
     RayRef32 r;
     if (MODE != INTERP_TRILINEAR) r = ray_ref32(g, p, v, u);
     const cudaTextureObject_t* tx = AX == 0 ? xtex : ytex;

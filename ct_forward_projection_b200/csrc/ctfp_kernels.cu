@@ -195,6 +195,65 @@ __global__ void __launch_bounds__(256, MINB) k_forward_axis(const MarchParams pr
     }
 }
 
+// K1+K2 with the axis sampler for a plan of few rays (axis_split), where a
+// thread per ray leaves most of the chip idle and the time is one ray's chain
+// of gathers: 1 << shift lanes share a ray, each marching an equal run of its
+// samples and taking a fourth of the energies.  A warp covers 32 >> shift rows
+// of one column (lane quads down 4 rows, as k_forward_axis), a CTA 4 columns.
+// The energies' partial sums are spectral()'s four accumulators, combined in
+// its order, so I and IAbs equal its values for the same L.
+template <int M, int MODE, bool SKIP, bool SPECTRAL>
+__global__ void __launch_bounds__(128, 8) k_forward_axis_split(const MarchParams prm, int shift)
+{
+    extern __shared__ float s_mu[];
+    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E * M);
+    const int lane = threadIdx.x & 31, rows = 32 >> shift, part = lane / rows;
+    const int u = blockIdx.x * 4 + (threadIdx.x >> 5), v = blockIdx.y * rows + lane % rows;
+    const int p = prm.view0 + blockIdx.z;
+    const bool on = u < prm.g.U && v < prm.g.V;
+    const int64_t npix = (int64_t)prm.g.U * prm.g.V;
+    const int64_t pix = (int64_t)v * prm.g.U + u;
+    const int64_t ray = (int64_t)(p - prm.out_view0) * npix + pix;
+    float L[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) L[m] = 0.f;
+    if (on) {
+        const OccView ov{prm.occ, prm.occ_x, prm.occ_y, prm.g.nx, prm.g.ny, prm.g.nz, kOccShift};
+        if (axis_is_x(prm.g, p)) march_ray_axis<M, MODE, 0, SKIP>(prm.g, prm.xtex, prm.ytex, ov, p, v, u, L, part, 1 << shift);
+        else march_ray_axis<M, MODE, 1, SKIP>(prm.g, prm.xtex, prm.ytex, ov, p, v, u, L, part, 1 << shift);
+    }
+    for (int d = rows; d < 32; d <<= 1)
+#pragma unroll
+        for (int m = 0; m < M; m++) L[m] += __shfl_xor_sync(0xffffffffu, L[m], d);
+    if (on && part == 0 && prm.L) store_L<M>(prm.L, ray, L);
+    if (SPECTRAL) {
+        // accumulators of this lane: two of the four (2 lanes per ray) or one
+        const int first = shift == 1 ? 2 * part : part, own = shift == 1 ? 2 : 1;
+        float sI = 0.f, sA = 0.f;
+        if (on && first < 4) {
+            const float* Wp = prm.W + pix;
+            const int E4 = prm.E & ~3;
+            for (int a = 0; a < own; a++) {
+                float tI = 0.f, tA = 0.f;
+#pragma unroll 4
+                for (int e = first + a; e < E4; e += 4) spectral_term<M>(s_mu, e, Wp, npix, L, tI, tA);
+                if (first + a == 0)
+                    for (int e = E4; e < prm.E; e++) spectral_term<M>(s_mu, e, Wp, npix, L, tI, tA);
+                sI += tI;
+                sA += tA;
+            }
+        }
+        for (int d = rows; d < 4 * rows / own; d <<= 1) {
+            sI += __shfl_xor_sync(0xffffffffu, sI, d);
+            sA += __shfl_xor_sync(0xffffffffu, sA, d);
+        }
+        if (on && part == 0) {
+            if (prm.I) prm.I[ray] = sI;
+            if (prm.IAbs) prm.IAbs[ray] = sA;
+        }
+    }
+}
+
 // Texture quad-gathers of the axis march (count_ray_axis) over every view,
 // with k_forward_axis's CTA tile and lane layout; out[0] += quads, out[1] +=
 // samples.  Grid: x = pixel tiles along u, y = along v, z = views.
@@ -978,6 +1037,45 @@ cudaError_t bwd_launch(const MarchParams& prm, const BwdGrid& b, cudaStream_t st
     return cudaGetLastError();
 }
 
+// log2 of the lanes per ray of a plan's march: 0 is k_forward_axis, one thread
+// per ray.  It depends on the plan's rays alone, so that every call of a plan
+// (a range of its views, any launch shape) sums a ray the same way.  The chip
+// holds 150 k threads of the march at a time: below a few times that, a thread
+// per ray runs as long as its longest ray plus a nearly empty last wave.
+// Measured, us a forward with 1 / 2 / 4 / 8 lanes per ray (2 materials unless
+// noted): 15 k rays of 32^3 57 / - / 44 / 43, 16 k of 64^3 103 / - / 43 / 38, 66 k
+// of 128^3 221 / - / 99 / 97, 144 k of 96^3 191 / - / 128 / 141, 393 k of 128^3
+// 367 / - / 308 / 346, 655 k of 128^3 531 / 453 / 473, 819 k of 64^3 365 / 398 /
+// 386, 1.0 M of 128^3 743 / 694 / 732 and (128 rows more) 690 / 678 / 697.
+int axis_split(const GeomParams& g)
+{
+    const int64_t rays = (int64_t)g.U * g.V * g.P;
+    return rays <= 20000 ? 3 : rays <= 400000 ? 2 : rays <= 700000 ? 1 : 0;
+}
+
+template <int M, int MODE, bool SKIP>
+cudaError_t split_launch(const MarchParams& prm, bool spec, int shift, cudaStream_t st)
+{
+    const size_t smem = spec ? sizeof(float) * (size_t)prm.E * M : 0;
+    const int rows = 32 >> shift;
+    const dim3 grid((prm.g.U + 3) / 4, (prm.g.V + rows - 1) / rows, prm.n_views);
+    if (grid.x == 0 || grid.y == 0 || grid.z == 0) return cudaSuccess;
+    if (spec) k_forward_axis_split<M, MODE, SKIP, true><<<grid, 128, smem, st>>>(prm, shift);
+    else k_forward_axis_split<M, MODE, SKIP, false><<<grid, 128, smem, st>>>(prm, shift);
+    return cudaGetLastError();
+}
+
+template <int M>
+cudaError_t split_dispatch(const MarchParams& prm, int interp, bool spec, int shift, cudaStream_t st)
+{
+    const bool skip = prm.occ != nullptr;
+    if (interp == INTERP_TRILINEAR)
+        return skip ? split_launch<M, INTERP_TRILINEAR, true>(prm, spec, shift, st)
+                    : split_launch<M, INTERP_TRILINEAR, false>(prm, spec, shift, st);
+    return skip ? split_launch<M, INTERP_TEXEMU, true>(prm, spec, shift, st)
+                : split_launch<M, INTERP_TEXEMU, false>(prm, spec, shift, st);
+}
+
 template <int M>
 cudaError_t bwd_dispatch(const MarchParams& prm, int interp, bool from_gL, const BwdGrid& b, cudaStream_t st)
 {
@@ -1015,6 +1113,16 @@ cudaError_t launch_forward_once(const MarchParams& prm, int M, int interp, int s
             case 2: return brick_dispatch<2>(prm, interp, do_spectral, maps, grid, smem, smem_tma, st);
             case 3: return brick_dispatch<3>(prm, interp, do_spectral, maps, grid, smem, smem_tma, st);
             case 4: return brick_dispatch<4>(prm, interp, do_spectral, maps, grid, smem, smem_tma, st);
+        }
+        return cudaErrorInvalidValue;
+    }
+    if (sampler == SAMPLER_AXIS && interp != INTERP_TEXTURE && axis_split(prm.g) > 0) {
+        const int shift = axis_split(prm.g);
+        switch (M) {
+            case 1: return split_dispatch<1>(prm, interp, do_spectral, shift, st);
+            case 2: return split_dispatch<2>(prm, interp, do_spectral, shift, st);
+            case 3: return split_dispatch<3>(prm, interp, do_spectral, shift, st);
+            case 4: return split_dispatch<4>(prm, interp, do_spectral, shift, st);
         }
         return cudaErrorInvalidValue;
     }
@@ -1057,7 +1165,8 @@ cudaError_t launch_forward(const MarchParams& prm_in, int M, int interp, int sam
                            const LaunchShape& ls, cudaStream_t st)
 {
     // view groups run along grid.z, at most 65535 per launch
-    const int vpc = ls.views_per_cta;
+    const bool split = sampler == SAMPLER_AXIS && interp != INTERP_TEXTURE && axis_split(prm_in.g) > 0;
+    const int vpc = split ? 1 : ls.views_per_cta;
     const int max_views = 65535 * vpc;
     for (int v0 = 0; v0 < prm_in.n_views; v0 += max_views) {
         MarchParams prm = prm_in;
