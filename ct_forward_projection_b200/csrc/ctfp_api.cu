@@ -2,7 +2,7 @@
 //
 // Ownership: the caller owns every buffer it passes (volumes, outputs,
 // checkpoints, gradients).  A plan owns its tables (view trigonometry, energy
-// weights W[E][V][U], flat field I0, attenuation table) and, in texture mode,
+// weights W, flat field I0, attenuation table) and, in texture mode,
 // one cudaArray + texture object per material.  No call resets the device and
 // none exits: every failure is a ctfp_status plus a per-thread message.
 #include <algorithm>
@@ -32,7 +32,7 @@ struct ctfp_plan {
     int E = 0;
     bool spectral_ready = false;
     float* d_mu = nullptr;  // [E][M]
-    float* d_W = nullptr;   // [E][V][U]
+    float* d_W = nullptr;   // energy weights (weight_index)
     float* d_I0 = nullptr;  // [V][U]
     // texture mode
     cudaArray_t arr[kMaxM] = {};
@@ -635,7 +635,7 @@ ctfp_status ctfp_set_spectral_tables(ctfp_plan* p, int32_t E, const float* spect
     cudaFree(p->d_I0); p->d_I0 = nullptr;
     p->spectral_ready = false;
     cudaError_t e = cudaMalloc(&p->d_mu, sizeof(float) * (size_t)E * p->M);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_W, sizeof(float) * (size_t)E * npix);
+    if (e == cudaSuccess) e = cudaMalloc(&p->d_W, sizeof(float) * weight_floats((int)U, (int)V, E));
     if (e == cudaSuccess) e = cudaMalloc(&p->d_I0, sizeof(float) * (size_t)npix);
     if (e == cudaSuccess) e = cudaMalloc(&dS, sizeof(float) * (size_t)E);
     if (e == cudaSuccess && nG) e = cudaMalloc(&dG, sizeof(float) * nG);

@@ -77,7 +77,7 @@ struct ItemDesc {
     cudaTextureObject_t ytex[kMaxM];
     cudaTextureObject_t tex[kMaxM];    // 3D textures (TEXTURE: the reference's own sampler)
     const float* mu;   // [E][M]
-    const float* W;    // [E][V][U]
+    const float* W;    // energy weights (weight_index)
     int M, E, interp;
     int tiles_u, tiles_v;
     int vgroups;       // groups of views per unit: ceil(P / views per unit)
@@ -221,7 +221,7 @@ __device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M
     if (!ADJOINT) {
         batch_march<M, MODE, AXIS>(it, tx, p, v, u, L);
         float I, A;
-        spectral<M>(s_mu, it.E, it.W, pix, npix, L, I, A);
+        spectral<M>(s_mu, it.E, pixel_weights(it.W, it.g.U, it.E, u, v), L, I, A);
         if (it.I) it.I[ray] = I;
         if (it.IAbs) it.IAbs[ray] = A;
         if (it.L) {
@@ -237,7 +237,7 @@ __device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M
     if (on) {
         batch_march<M, MODE, AXIS>(it, tx, p, v, u, L);
         float I, S[M];
-        spectral_adjoint<M>(s_mu, it.E, it.W, pix, npix, L, I, S);
+        spectral_adjoint<M>(s_mu, it.E, pixel_weights(it.W, it.g.U, it.E, u, v), L, I, S);
         if (it.I) it.I[ray] = I;
         // loss (log I - log T)^2: dLoss/dI = 2 (log I - log T) / I, dI/dL_m = -S_m
         if (I > 0.f) {
@@ -254,7 +254,7 @@ __device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M
     // emulation reproduces exactly (as ctfp_backward does for such a plan)
     constexpr int SM = MODE == INTERP_TRILINEAR ? INTERP_TRILINEAR : INTERP_TEXEMU;
     if (!AXIS && !it.gcol) scatter_direct<M, SM>(it.g, it.gvol, any, p, v, u, g);
-    else scatter_columns<M, SM>(it.g, it.gcol + (size_t)set * it.set_floats, any, p, v, u, g);
+    else scatter_columns<M, SM, (M > 2 && MODE == INTERP_TRILINEAR)>(it.g, it.gcol + (size_t)set * it.set_floats, any, p, v, u, g);
     return res * res;
 }
 
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJO
     k_batch(const GroupArgs a)
 {
     constexpr int kThreads = BatchShape<ADJOINT>::threads, kWarps = BatchShape<ADJOINT>::warps;
-    __shared__ float s_mu[CTFP_MAX_ENERGIES * M];
+    __shared__ __align__(16) float s_mu[CTFP_MAX_ENERGIES * M];
     __shared__ float s_loss[kWarps];
     // the current unit as thread 0 decoded it: item, first view, tile column
     // and row, and whether the item changed.  Every thread re-reads these
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJO
         if (*(volatile int*)&s_end) break;
         const ItemDesc* const itp = a.items + *(volatile int*)&s_item;
         if (*(volatile int*)&s_new) {
-            for (int j = threadIdx.x; j < itp->E * M; j += kThreads) s_mu[j] = itp->mu[j];
+            stage_mu(s_mu, itp->mu, itp->E, M, threadIdx.x, kThreads);
             __syncthreads();
         }
         const ItemTex<M> tx = item_tex<M, MODE, AXIS>(*itp);

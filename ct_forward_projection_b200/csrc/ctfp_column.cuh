@@ -156,11 +156,11 @@ __device__ __forceinline__ void red_v4_if(bool on, float* q, float a, float b, f
 // One ray's face sums on their way into memory: slot 0 the even layer, slot 1
 // the odd one of its current pair, each the summed weights of (a, b),
 // (a + 1, b), (a, b + 1), (a + 1, b + 1); a slot is flushed when its layer or
-// the in-layer base changes.  Above two materials the whole warp calls move()
-// and finish() together.
-template <int M>
+// the in-layer base changes.  MERGE: the whole warp calls move() and finish()
+// together.
+template <int M, bool MERGE>
 struct ColumnScatter {
-    static constexpr bool warp_wide = M > 2;
+    static constexpr bool warp_wide = MERGE;
     float* acc;
     const float* g;  // dLoss/dL_m times dx
     unsigned sA;
@@ -178,15 +178,21 @@ struct ColumnScatter {
         for (int j = 0; j < 4; j++) s0[j] = s1[j] = 0.f;
     }
 
-    // Pair cells, one lane on its own.
+    // One lane on its own.
     __device__ __forceinline__ void flush_cells(unsigned at, const float* s) const
     {
         constexpr int W = accum_width(M);
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             float* q = acc + (size_t)(at + (c ? sA : 0u)) * W;
-            if (M == 1) red_v2(q, s[c] * g[0], s[c + 2] * g[0]);
-            else red_v4(q, s[c] * g[0], s[c] * g[M - 1], s[c + 2] * g[0], s[c + 2] * g[M - 1]);
+            if (M == 1) {
+                red_v2(q, s[c] * g[0], s[c + 2] * g[0]);
+            } else if (M == 2) {
+                red_v4(q, s[c] * g[0], s[c] * g[M - 1], s[c + 2] * g[0], s[c + 2] * g[M - 1]);
+            } else {
+                red_v4(q, s[c] * g[0], s[c] * g[1 % M], s[c] * g[2 % M], M == 4 ? s[c] * g[M - 1] : 0.f);
+                red_v4(q + W, s[c + 2] * g[0], s[c + 2] * g[1 % M], s[c + 2] * g[2 % M], M == 4 ? s[c + 2] * g[M - 1] : 0.f);
+            }
         }
     }
 
@@ -222,7 +228,7 @@ struct ColumnScatter {
 
     __device__ __forceinline__ void flush(bool need, unsigned at, const float* s) const
     {
-        if (M > 2) flush_voxels(need, at, s);
+        if (MERGE) flush_voxels(need, at, s);
         else if (need) flush_cells(at, s);
     }
 
@@ -254,7 +260,7 @@ struct ColumnScatter {
     }
 };
 
-template <int M>
+template <int M, bool MERGE>
 __device__ __forceinline__ void scatter_trilinear(const GeomParams& gp, float* acc, bool on, int p, int v, int u,
                                                   const float* g)
 {
@@ -265,7 +271,7 @@ __device__ __forceinline__ void scatter_trilinear(const GeomParams& gp, float* a
     const double i0 = (double)s.i0;
     double cl = fma(i0, bl, xl ? s.ax : s.ay), ca = fma(i0, ba, xl ? s.ay : s.ax), cz = fma(i0, bz, s.az);
     const unsigned sL = xl ? cd.sx : cd.sy, sA = xl ? cd.sy : cd.sx;
-    using Scatter = ColumnScatter<M>;
+    using Scatter = ColumnScatter<M, MERGE>;
     const int n = on ? s.i1 - s.i0 : 0, steps = Scatter::steps(n);
     Scatter k;
     k.begin(acc, g, sA);
@@ -291,7 +297,7 @@ __device__ __forceinline__ void scatter_trilinear(const GeomParams& gp, float* a
     k.finish();
 }
 
-template <int M, bool XL>
+template <int M, bool MERGE, bool XL>
 __device__ __forceinline__ void scatter_texemu(const GeomParams& gp, float* acc, bool on, int p, int v, int u,
                                                const float* g)
 {
@@ -299,7 +305,7 @@ __device__ __forceinline__ void scatter_texemu(const GeomParams& gp, float* acc,
     const RayRef32 r = ray_ref32(gp, p, v, u);
     const ColumnDims cd = column_dims(gp.nx, gp.ny, gp.nz);
     const unsigned sL = XL ? cd.sx : cd.sy, sA = XL ? cd.sy : cd.sx;
-    using Scatter = ColumnScatter<M>;
+    using Scatter = ColumnScatter<M, MERGE>;
     const int n = on ? s.i1 - s.i0 : 0, steps = Scatter::steps(n);
     Scatter k;
     k.begin(acc, g, sA);
@@ -327,14 +333,14 @@ __device__ __forceinline__ void scatter_texemu(const GeomParams& gp, float* acc,
 
 // The adjoint of one ray's march, scaled by g[m] = dLoss/dL_m times dx, for
 // the lanes with on set; every lane of the warp calls it, for the same view.
-template <int M, int MODE>
+template <int M, int MODE, bool MERGE>
 __device__ __forceinline__ void scatter_columns(const GeomParams& gp, float* acc, bool on, int p, int v, int u,
                                                 const float* g)
 {
-    if (!ColumnScatter<M>::warp_wide && !on) return;
-    if (MODE == INTERP_TRILINEAR) scatter_trilinear<M>(gp, acc, on, p, v, u, g);
-    else if (axis_is_x(gp, p)) scatter_texemu<M, true>(gp, acc, on, p, v, u, g);
-    else scatter_texemu<M, false>(gp, acc, on, p, v, u, g);
+    if (!MERGE && !on) return;
+    if (MODE == INTERP_TRILINEAR) scatter_trilinear<M, MERGE>(gp, acc, on, p, v, u, g);
+    else if (axis_is_x(gp, p)) scatter_texemu<M, MERGE, true>(gp, acc, on, p, v, u, g);
+    else scatter_texemu<M, MERGE, false>(gp, acc, on, p, v, u, g);
 }
 
 // The same for a volume that column_fits refuses: every voxel of every sample

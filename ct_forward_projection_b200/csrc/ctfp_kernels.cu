@@ -92,10 +92,9 @@ __device__ __forceinline__ void march_ray(const MarchParams& prm, int p, int v, 
     for (int m = 0; m < M; m++) L[m] = prm.g.dx * (acc[m] - cmp[m]);
 }
 
-__device__ __forceinline__ void load_mu(float* s_mu, const float* mu, int n)
+__device__ __forceinline__ void load_mu(float* s_mu, const float* mu, int E, int M)
 {
-    const int nt = blockDim.x * blockDim.y;
-    for (int k = threadIdx.y * blockDim.x + threadIdx.x; k < n; k += nt) s_mu[k] = mu[k];
+    stage_mu(s_mu, mu, E, M, threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y);
     __syncthreads();
 }
 
@@ -133,8 +132,8 @@ __device__ __forceinline__ void load_L(const float* L, int64_t ray, float* l)
 template <int M, int MODE, int SAMPLER, bool SPECTRAL, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_forward(const MarchParams prm)
 {
-    extern __shared__ float s_mu[];
-    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E * M);
+    extern __shared__ __align__(16) float s_mu[];
+    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E, M);
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     const int v = blockIdx.y * blockDim.y + threadIdx.y;
     if (u >= prm.g.U || v >= prm.g.V) return;
@@ -150,7 +149,7 @@ __global__ void __launch_bounds__(256, MINB) k_forward(const MarchParams prm)
         if (prm.L) store_L<M>(prm.L, ray, L);
         if (SPECTRAL) {
             float I, A;
-            spectral<M>(s_mu, prm.E, prm.W, pix, npix, L, I, A);
+            spectral<M>(s_mu, prm.E, pixel_weights(prm.W, prm.g.U, prm.E, u, v), L, I, A);
             if (prm.I) prm.I[ray] = I;
             if (prm.IAbs) prm.IAbs[ray] = A;
         }
@@ -164,8 +163,8 @@ __global__ void __launch_bounds__(256, MINB) k_forward(const MarchParams prm)
 template <int M, int MODE, bool SKIP, bool SPECTRAL, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_forward_axis(const MarchParams prm, int tile_u, int warp_rows)
 {
-    extern __shared__ float s_mu[];
-    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E * M);
+    extern __shared__ __align__(16) float s_mu[];
+    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E, M);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int tile_v = (int)blockDim.x / tile_u;
     // a warp covers wcols columns x warp_rows rows, lane quads down 4 rows
@@ -188,7 +187,7 @@ __global__ void __launch_bounds__(256, MINB) k_forward_axis(const MarchParams pr
         if (prm.L) store_L<M>(prm.L, ray, L);
         if (SPECTRAL) {
             float I, A;
-            spectral<M>(s_mu, prm.E, prm.W, pix, npix, L, I, A);
+            spectral<M>(s_mu, prm.E, pixel_weights(prm.W, prm.g.U, prm.E, u, v), L, I, A);
             if (prm.I) prm.I[ray] = I;
             if (prm.IAbs) prm.IAbs[ray] = A;
         }
@@ -205,8 +204,8 @@ __global__ void __launch_bounds__(256, MINB) k_forward_axis(const MarchParams pr
 template <int M, int MODE, bool SKIP, bool SPECTRAL>
 __global__ void __launch_bounds__(128, 8) k_forward_axis_split(const MarchParams prm, int shift)
 {
-    extern __shared__ float s_mu[];
-    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E * M);
+    extern __shared__ __align__(16) float s_mu[];
+    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E, M);
     const int lane = threadIdx.x & 31, rows = 32 >> shift, part = lane / rows;
     const int u = blockIdx.x * 4 + (threadIdx.x >> 5), v = blockIdx.y * rows + lane % rows;
     const int p = prm.view0 + blockIdx.z;
@@ -231,14 +230,23 @@ __global__ void __launch_bounds__(128, 8) k_forward_axis_split(const MarchParams
         const int first = shift == 1 ? 2 * part : part, own = shift == 1 ? 2 : 1;
         float sI = 0.f, sA = 0.f;
         if (on && first < 4) {
-            const float* Wp = prm.W + pix;
-            const int E4 = prm.E & ~3;
+            const float* Wp = (const float*)pixel_weights(prm.W, prm.g.U, prm.E, u, v);
+            const int full = prm.E >> 2, Ep = energy_groups(prm.E) * 4;
             for (int a = 0; a < own; a++) {
                 float tI = 0.f, tA = 0.f;
+                const auto term = [&](int e) {
+                    float att = 0.f, ex, om;
+#pragma unroll
+                    for (int m = 0; m < M; m++) att = fmaf(s_mu[m * Ep + e], L[m], att);
+                    const float w = __ldg(Wp + (e >> 2) * 128 + (e & 3));
+                    transmit(att, ex, om);
+                    tI = fmaf(w, ex, tI);
+                    tA = fmaf(w, om, tA);
+                };
 #pragma unroll 4
-                for (int e = first + a; e < E4; e += 4) spectral_term<M>(s_mu, e, Wp, npix, L, tI, tA);
+                for (int g = 0; g < full; g++) term(4 * g + first + a);
                 if (first + a == 0)
-                    for (int e = E4; e < prm.E; e++) spectral_term<M>(s_mu, e, Wp, npix, L, tI, tA);
+                    for (int e = 4 * full; e < prm.E; e++) term(e);
                 sI += tI;
                 sA += tA;
             }
@@ -316,20 +324,26 @@ __global__ void k_axis_zero_layer(cudaSurfaceObject_t sf, int width, int height,
         surf2DLayeredwrite(0.0f, sf, (k % width) * (int)sizeof(float), k / width, layer);
 }
 
+// K2 on stored line integrals; threads walk the views' pixels in W's block
+// order.
 template <int M>
 __global__ void __launch_bounds__(256) k_spectral_from_L(const MarchParams prm)
 {
-    extern __shared__ float s_mu[];
-    load_mu(s_mu, prm.mu, prm.E * M);
-    const int64_t npix = (int64_t)prm.g.U * prm.g.V;
-    const int64_t nray = npix * prm.g.P;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x * blockDim.y;
-    for (int64_t ray = (int64_t)blockIdx.x * blockDim.x * blockDim.y + threadIdx.y * blockDim.x + threadIdx.x;
-         ray < nray; ray += stride) {
+    extern __shared__ __align__(16) float s_mu[];
+    load_mu(s_mu, prm.mu, prm.E, M);
+    const int bu = (prm.g.U + 3) >> 2, bv = (prm.g.V + 7) >> 3;
+    const int64_t npix = (int64_t)prm.g.U * prm.g.V, per_view = (int64_t)bu * bv * 32;
+    const int64_t n = per_view * prm.g.P, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += stride) {
+        const int64_t p = t / per_view;
+        const int r = (int)(t - p * per_view), block = r >> 5, lane = r & 31;
+        const int u = (block % bu) * 4 + (lane & 3), v = (block / bu) * 8 + (lane >> 2);
+        if (u >= prm.g.U || v >= prm.g.V) continue;
+        const int64_t ray = p * npix + (int64_t)v * prm.g.U + u;
         float L[M];
         load_L<M>(prm.Lin, ray, L);
         float I, A;
-        spectral<M>(s_mu, prm.E, prm.W, ray % npix, npix, L, I, A);
+        spectral<M>(s_mu, prm.E, pixel_weights(prm.W, prm.g.U, prm.E, u, v), L, I, A);
         if (prm.I) prm.I[ray] = I;
         if (prm.IAbs) prm.IAbs[ray] = A;
     }
@@ -347,13 +361,15 @@ __global__ void __launch_bounds__(256) k_spectral_from_L(const MarchParams prm)
 // views outermost every view would sweep the whole accumulator through DRAM.
 // Register cap for 4 CTAs of 256 threads (64 registers): more warps hide the
 // reductions' latency.
-// DIRECT: no accumulators (prm.gcol null), the gradients take the sums.
-template <int M, int MODE, bool FROM_GL, bool DIRECT>
+// KIND: kEach, kMerge (merge_faces) or kDirect: no accumulators (prm.gcol null),
+// the gradients take the sums.
+enum { kEach, kMerge, kDirect };
+template <int M, int MODE, bool FROM_GL, int KIND>
 __global__ void __launch_bounds__(256, 4)
     k_backward(const MarchParams prm, int tile_u, int warp_rows, int tiles_v, int set_groups)
 {
-    extern __shared__ float s_mu[];
-    if (!FROM_GL) load_mu(s_mu, prm.mu, prm.E * M);
+    extern __shared__ __align__(16) float s_mu[];
+    if (!FROM_GL) load_mu(s_mu, prm.mu, prm.E, M);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int tile_v = (int)blockDim.x / tile_u;
     const int wcols = 32 / warp_rows, warps_u = tile_u / wcols;
@@ -384,16 +400,15 @@ __global__ void __launch_bounds__(256, 4)
                 for (int m = 0; m < M; m++) S[m] = 0.f;
                 // the spectral weights as the forward formed them (transmit, the
                 // same order), so S matches the fused kernels' exactly
-                for (int e = 0; e < prm.E; e++) {
-                    float att = 0.f;
+                const int Ep = energy_groups(prm.E) * 4;
+                for_energies<M>(s_mu, prm.E, pixel_weights(prm.W, prm.g.U, prm.E, u, v), L,
+                                [&](int, int e, float att, float wt) {
+                                    float ex, om;
+                                    transmit(att, ex, om);
+                                    const float Ie = wt * ex;
 #pragma unroll
-                    for (int m = 0; m < M; m++) att = fmaf(s_mu[e * M + m], L[m], att);
-                    float ex, om;
-                    transmit(att, ex, om);
-                    const float Ie = __ldg(prm.W + (int64_t)e * npix + pix) * ex;
-#pragma unroll
-                    for (int m = 0; m < M; m++) S[m] = fmaf(s_mu[e * M + m], Ie, S[m]);
-                }
+                                    for (int m = 0; m < M; m++) S[m] = fmaf(s_mu[m * Ep + e], Ie, S[m]);
+                                });
                 const float gd = ((prm.gIAbs ? prm.gIAbs[ray] : 0.f) - (prm.gI ? prm.gI[ray] : 0.f)) * prm.g.dx;
 #pragma unroll
                 for (int m = 0; m < M; m++) g[m] = gd * S[m];
@@ -404,8 +419,8 @@ __global__ void __launch_bounds__(256, 4)
         // the transposed weights of the forward's sampler (for the texture
         // modes, the texture unit's, at the reference's FP32 coordinates)
         constexpr int SM = MODE == INTERP_TRILINEAR ? INTERP_TRILINEAR : INTERP_TEXEMU;
-        if (DIRECT) scatter_direct<M, SM>(prm.g, prm.gvol, any, p, v, u, g);
-        else scatter_columns<M, SM>(prm.g, prm.gcol + (size_t)set * prm.set_floats, any, p, v, u, g);
+        if (KIND == kDirect) scatter_direct<M, SM>(prm.g, prm.gvol, any, p, v, u, g);
+        else scatter_columns<M, SM, KIND == kMerge>(prm.g, prm.gcol + (size_t)set * prm.set_floats, any, p, v, u, g);
     }
 }
 
@@ -421,30 +436,37 @@ __global__ void __launch_bounds__(256) k_fold(const MarchParams prm)
 }
 
 // W[e][k] = ((I0Val * S_e) * G_e) * D_e in the reference's multiplication order
-// (CBCTPolyProjGPU.cu:1994); I0[k] = the sum over e (CBCTPolyForwardProjGrid.cpp:330-339).
+// (CBCTPolyProjGPU.cu:1994), laid out as weight_index; I0[k] = the sum over e
+// (CBCTPolyForwardProjGrid.cpp:330-339).
 __global__ void k_weights(const float* __restrict__ S, const float* __restrict__ G, int grid_layout,
                           const float* __restrict__ D, float I0Val, int E, int U, int V, float* W, float* I0)
 {
     const int64_t npix = (int64_t)U * V;
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < npix; k += (int64_t)gridDim.x * blockDim.x) {
-        const int u = (int)(k % U);
+        const int u = (int)(k % U), v = (int)(k / U);
         // the spectral epilogue's summation order (energy e into accumulator
         // e mod 4, E rounded down to a multiple of 4 first, the rest into
         // accumulator 0, combined pairwise), so that a ray with no attenuation
         // gives exactly I0
         float s[4] = {0.f, 0.f, 0.f, 0.f};
-        const int E4 = E & ~3;
-        for (int e = 0; e < E; e++) {
-            float w = I0Val * S[e];
-            if (grid_layout == 1) w = w * G[(int64_t)e * U + u];
-            if (grid_layout == 2) w = w * G[(int64_t)e * npix + k];
-            if (D) w = w * D[(int64_t)e * npix + k];
-            W[(int64_t)e * npix + k] = w;
-            const int a = e < E4 ? (e & 3) : 0;
-            if (a == 0) s[0] += w;
-            else if (a == 1) s[1] += w;
-            else if (a == 2) s[2] += w;
-            else s[3] += w;
+        float4* Wp = (float4*)(W + weight_index(U, E, u, v));
+        const int E4 = energy_groups(E);
+        for (int g = 0; g < E4; g++) {
+            float w[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int e = 4 * g + j;
+                w[j] = 0.f;
+                if (e < E) {
+                    w[j] = I0Val * S[e];
+                    if (grid_layout == 1) w[j] = w[j] * G[(int64_t)e * U + u];
+                    if (grid_layout == 2) w[j] = w[j] * G[(int64_t)e * npix + k];
+                    if (D) w[j] = w[j] * D[(int64_t)e * npix + k];
+                    if (4 * g + 4 <= E) s[j] += w[j];
+                    else s[0] += w[j];
+                }
+            }
+            Wp[g * 32] = make_float4(w[0], w[1], w[2], w[3]);
         }
         I0[k] = (s[0] + s[1]) + (s[2] + s[3]);
     }
@@ -537,11 +559,11 @@ __device__ __forceinline__ Corner corner_at(const MarchParams& prm, const RaySeg
 template <int M, int MODE, bool SPECTRAL, int MINB>
 __global__ void __launch_bounds__(kBU * kBV, MINB) k_forward_brick(const MarchParams prm)
 {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     float* s_box = smem;                   // [M][kBZ][kBY][kBXp] (slices kBZp apart)
     float* s_mu = smem + M * kBoxFloats;   // [E][M]
     __shared__ int s_red[8];
-    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E * M);
+    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E, M);
     const int tid = threadIdx.y * kBU + threadIdx.x;
     const int u = blockIdx.x * kBU + threadIdx.x;
     const int v = blockIdx.y * kBV + threadIdx.y;
@@ -638,7 +660,7 @@ __global__ void __launch_bounds__(kBU * kBV, MINB) k_forward_brick(const MarchPa
         if (prm.L) store_L<M>(prm.L, ray, L);
         if (SPECTRAL) {
             float I, A;
-            spectral<M>(s_mu, prm.E, prm.W, pix, npix, L, I, A);
+            spectral<M>(s_mu, prm.E, pixel_weights(prm.W, prm.g.U, prm.E, u, v), L, I, A);
             if (prm.I) prm.I[ray] = I;
             if (prm.IAbs) prm.IAbs[ray] = A;
         }
@@ -727,7 +749,7 @@ __global__ void __launch_bounds__(kBU * kBV, MINB)
     __shared__ __align__(8) uint64_t s_bar;
     const int tid = threadIdx.y * kBU + threadIdx.x;
     if (tid == 0) mbar_init(&s_bar, 1);
-    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E * M);
+    if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E, M);
     __syncthreads();
     uint32_t phase = 0;
     bool staging = true;   // CTA-uniform: false once a wait ran out
@@ -831,7 +853,7 @@ __global__ void __launch_bounds__(kBU * kBV, MINB)
         if (prm.L) store_L<M>(prm.L, ray, L);
         if (SPECTRAL) {
             float I, A;
-            spectral<M>(s_mu, prm.E, prm.W, pix, npix, L, I, A);
+            spectral<M>(s_mu, prm.E, pixel_weights(prm.W, prm.g.U, prm.E, u, v), L, I, A);
             if (prm.I) prm.I[ray] = I;
             if (prm.IAbs) prm.IAbs[ray] = A;
         }
@@ -1022,6 +1044,21 @@ cudaError_t axis_dispatch(const MarchParams& prm, int interp, bool spec, int min
     return cudaErrorInvalidValue;
 }
 
+// Whether the scatter of three or four materials hands sums over between rows
+// (flush_voxels): the shuffles pay while neighbouring rows mostly flush
+// neighbouring voxels, and for the texture emulation, whose samples cost more
+// instructions, only where the L2's reductions bind.  Measured, adjoint + fold,
+// each lane on its own / merged, ms -- trilinear, 3 materials: 64^3, row
+// spacing 1.3 voxels 0.392 / 0.346, 176^3, 1.0 5.69 / 4.37, 128^3, 2.0 1.00 / 1.08;
+// texture emulation: 96^3, 1.0 1.03 / 1.06, 128^3, 0.5 3.76 / 3.22, 256^3, 1.3
+// 9.47 / 8.66, 128^3, 2.0 1.03 / 1.13.
+bool merge_faces(const GeomParams& g, int interp)
+{
+    const float rows = g.dSize * g.sod / (g.sdd * g.pSizeZ);
+    if (rows >= 1.8f) return false;
+    return interp == INTERP_TRILINEAR || rows < 0.7f || (int64_t)g.nx * g.ny * g.nz > 2000000;
+}
+
 struct BwdGrid {
     int tile_u, rows, tiles_v, set_groups;
     dim3 grid, block;
@@ -1032,7 +1069,9 @@ template <int M, int MODE, bool FROM_GL>
 cudaError_t bwd_launch(const MarchParams& prm, const BwdGrid& b, cudaStream_t st)
 {
     const size_t smem = FROM_GL ? 0 : b.smem;
-    const auto k = prm.gcol ? k_backward<M, MODE, FROM_GL, false> : k_backward<M, MODE, FROM_GL, true>;
+    auto k = k_backward<M, MODE, FROM_GL, kEach>;
+    if (!prm.gcol) k = k_backward<M, MODE, FROM_GL, kDirect>;
+    else if (M > 2 && merge_faces(prm.g, MODE)) k = k_backward<M, MODE, FROM_GL, (M > 2 ? kMerge : kEach)>;
     k<<<b.grid, b.block, smem, st>>>(prm, b.tile_u, b.rows, b.tiles_v, b.set_groups);
     return cudaGetLastError();
 }
@@ -1056,7 +1095,7 @@ int axis_split(const GeomParams& g)
 template <int M, int MODE, bool SKIP>
 cudaError_t split_launch(const MarchParams& prm, bool spec, int shift, cudaStream_t st)
 {
-    const size_t smem = spec ? sizeof(float) * (size_t)prm.E * M : 0;
+    const size_t smem = spec ? sizeof(float) * (size_t)energy_groups(prm.E) * 4 * M : 0;
     const int rows = 32 >> shift;
     const dim3 grid((prm.g.U + 3) / 4, (prm.g.V + rows - 1) / rows, prm.n_views);
     if (grid.x == 0 || grid.y == 0 || grid.z == 0) return cudaSuccess;
@@ -1103,7 +1142,7 @@ cudaError_t launch_forward_once(const MarchParams& prm, int M, int interp, int s
         const dim3 grid((prm.g.U + kBU - 1) / kBU, (prm.g.V + kBV - 1) / kBV,
                         (prm.n_views + ls.views_per_cta - 1) / ls.views_per_cta);
         if (grid.z == 0) return cudaSuccess;
-        const size_t mu_floats = do_spectral ? (size_t)prm.E * M : 0;
+        const size_t mu_floats = do_spectral ? (size_t)energy_groups(prm.E) * 4 * M : 0;
         const size_t smem = sizeof(float) * ((size_t)M * kBoxFloats + mu_floats);
         const size_t smem_tma = 128 + sizeof(float) * ((size_t)M * kTBoxFloats + mu_floats);  // + alignment slack
         BrickMaps bm;
@@ -1137,7 +1176,7 @@ cudaError_t launch_forward_once(const MarchParams& prm, int M, int interp, int s
             as.tile_v = 16;
         }
         const dim3 block(as.tile_u * as.tile_v), grid = march_grid(prm, as);
-        const size_t smem = do_spectral ? sizeof(float) * (size_t)prm.E * M : 0;
+        const size_t smem = do_spectral ? sizeof(float) * (size_t)energy_groups(prm.E) * 4 * M : 0;
         if (grid.x == 0 || grid.y == 0 || grid.z == 0) return cudaSuccess;
         switch (M) {
             case 1: return axis_dispatch<1>(prm, interp, do_spectral, as.min_ctas, as.tile_u, grid, block, smem, st);
@@ -1148,7 +1187,7 @@ cudaError_t launch_forward_once(const MarchParams& prm, int M, int interp, int s
         return cudaErrorInvalidValue;
     }
     const dim3 block(ls.tile_u, ls.tile_v), grid = march_grid(prm, ls);
-    const size_t smem = do_spectral ? sizeof(float) * (size_t)prm.E * M : 0;
+    const size_t smem = do_spectral ? sizeof(float) * (size_t)energy_groups(prm.E) * 4 * M : 0;
     if (grid.x == 0 || grid.y == 0 || grid.z == 0) return cudaSuccess;
     switch (M) {
         case 1: return fwd_dispatch_mode<1>(prm, interp, sampler, do_spectral, ls.min_ctas, grid, block, smem, st);
@@ -1228,11 +1267,11 @@ cudaError_t launch_axis_fill(const float* vol, int nx, int ny, int nz, cudaSurfa
 cudaError_t launch_spectral_from_L(const MarchParams& prm, int M, cudaStream_t st)
 {
     const dim3 block(256, 1);
-    const int64_t nray = (int64_t)prm.g.U * prm.g.V * prm.g.P;
-    int64_t nb = (nray + 255) / 256;
+    const int64_t n = (int64_t)((prm.g.U + 3) / 4) * ((prm.g.V + 7) / 8) * 32 * prm.g.P;
+    int64_t nb = (n + 255) / 256;
     if (nb > 148 * 64) nb = 148 * 64;
     if (nb == 0) return cudaSuccess;
-    const size_t smem = sizeof(float) * (size_t)prm.E * M;
+    const size_t smem = sizeof(float) * (size_t)energy_groups(prm.E) * 4 * M;
     switch (M) {
         case 1: k_spectral_from_L<1><<<(unsigned)nb, block, smem, st>>>(prm); break;
         case 2: k_spectral_from_L<2><<<(unsigned)nb, block, smem, st>>>(prm); break;
@@ -1273,7 +1312,7 @@ cudaError_t launch_backward(const MarchParams& prm_in, int M, int interp, bool f
     b.rows = rows;
     b.tiles_v = (prm_in.g.V + bs.tile_v - 1) / bs.tile_v;
     b.block = dim3(threads);
-    b.smem = sizeof(float) * (size_t)prm_in.E * M;
+    b.smem = sizeof(float) * (size_t)energy_groups(prm_in.E) * 4 * M;
     const unsigned tiles_u = (unsigned)((prm_in.g.U + bs.tile_u - 1) / bs.tile_u);
     // view groups run along grid.y, at most 65535 per launch: all sets in one
     // launch, or past that one part of a set's views after the other
