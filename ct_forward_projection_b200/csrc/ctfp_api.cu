@@ -45,6 +45,7 @@ struct ctfp_plan {
     cudaArray_t xarr[kMaxM] = {}, yarr[kMaxM] = {};
     cudaTextureObject_t xtex[kMaxM] = {}, ytex[kMaxM] = {};
     cudaSurfaceObject_t xsurf[kMaxM] = {}, ysurf[kMaxM] = {};
+    float* d_cvol = nullptr;  // the same for four materials: one column copy (ctfp_column.cuh)
     LaunchShape shape{};
     unsigned long long* d_count = nullptr;
     // empty-space skipping (off by default): brick occupancy, rebuilt from the
@@ -254,6 +255,14 @@ ctfp_status make_layered_rw(size_t width, size_t height, size_t layers, cudaArra
 ctfp_status make_axis(ctfp_plan* p)
 {
     const size_t nx = (size_t)p->geom.pNumX, ny = (size_t)p->geom.pNumY, nz = (size_t)p->geom.pNumZ;
+    if (axis_uses_columns(p->M)) {
+        if (p->d_cvol) return CTFP_OK;
+        const size_t bytes = sizeof(float) * column_floats((int)nx, (int)ny, (int)nz);
+        CTFP_CUDA(cudaMalloc(&p->d_cvol, bytes));
+        CTFP_CUDA(cudaMemset(p->d_cvol, 0, bytes));
+        CTFP_CUDA(cudaStreamSynchronize(0));
+        return CTFP_OK;
+    }
     for (int m = 0; m < p->M; m++) {
         if (p->xarr[m]) continue;
         ctfp_status st = make_layered_rw(ny, nz, nx + 2, p->xarr[m], p->xtex[m], p->xsurf[m]);
@@ -299,6 +308,10 @@ bool uses_axis(const ctfp_plan* p) { return p->interp != INTERP_TEXTURE && p->sa
 ctfp_status upload_textures(ctfp_plan* p, const float* const* volumes, cudaStream_t st)
 {
     const bool tex3d = p->interp == INTERP_TEXTURE;
+    if (uses_axis(p) && axis_uses_columns(p->M)) {
+        CTFP_CUDA(launch_column_fill(volumes, (int)p->geom.pNumX, (int)p->geom.pNumY, (int)p->geom.pNumZ, p->d_cvol, st));
+        return CTFP_OK;
+    }
     if (uses_axis(p)) {
         for (int m = 0; m < p->M; m++)
             CTFP_CUDA(launch_axis_fill(volumes[m], (int)p->geom.pNumX, (int)p->geom.pNumY, (int)p->geom.pNumZ,
@@ -345,6 +358,7 @@ MarchParams base_params(const ctfp_plan* p)
         prm.xtex[m] = p->xtex[m];
         prm.ytex[m] = p->ytex[m];
     }
+    prm.cvol = p->d_cvol;
     if (p->skip_empty && p->d_occ) {
         prm.occ = p->d_occ;
         prm.occ_x = occ_dim(p->gp.nx);
@@ -491,6 +505,9 @@ ctfp_status ctfp_plan_create(const ctfp_geometry* g, int32_t n_materials, int32_
     p->M = n_materials;
     p->interp = interp;
     p->device = device;
+    // the column march holds 32 corner values per ray: 80 registers instead of
+    // 64 (512^3, 48 views: 145 against 184 ms)
+    if (axis_uses_columns(n_materials)) p->shape.min_ctas = 3;
     GeomParams& gp = p->gp;
     gp.nx = (int)g->pNumX; gp.ny = (int)g->pNumY; gp.nz = (int)g->pNumZ;
     gp.U = (int)g->dNumU; gp.V = (int)g->dNumV; gp.P = (int)g->projNum;
@@ -559,6 +576,7 @@ ctfp_status ctfp_plan_destroy(ctfp_plan* p)
     cudaFree(p->d_count);
     for (int m = 0; m < kMaxM; m++) cudaFree(p->h2d_vol[m]);
     cudaFree(p->d_gcol);
+    cudaFree(p->d_cvol);
     cudaFree(p->d_occ);
     cudaFree(p->d_status);
     for (cudaEvent_t& e : p->chunk_done)
@@ -982,6 +1000,7 @@ LaunchShape& plan_shape(ctfp_plan* p) { return p->shape; }
 cudaTextureObject_t plan_ltex(const ctfp_plan* p, int m) { return p->ltex[m]; }
 cudaTextureObject_t plan_xtex(const ctfp_plan* p, int m) { return p->xtex[m]; }
 cudaTextureObject_t plan_ytex(const ctfp_plan* p, int m) { return p->ytex[m]; }
+const float* plan_cvol(const ctfp_plan* p) { return p->d_cvol; }
 cudaTextureObject_t plan_tex(const ctfp_plan* p, int m) { return p->tex[m]; }
 MarchParams plan_march_params(const ctfp_plan* p) { return base_params(p); }
 const ctfp_geometry& plan_geometry(const ctfp_plan* p) { return p->geom; }

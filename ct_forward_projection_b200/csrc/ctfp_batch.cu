@@ -43,6 +43,7 @@ cudaTextureObject_t plan_ltex(const ctfp_plan* p, int m);
 cudaTextureObject_t plan_xtex(const ctfp_plan* p, int m);
 cudaTextureObject_t plan_ytex(const ctfp_plan* p, int m);
 cudaTextureObject_t plan_tex(const ctfp_plan* p, int m);
+const float* plan_cvol(const ctfp_plan* p);
 ctfp_status plan_upload(ctfp_plan* p, const float* const* volumes, cudaStream_t st);
 }  // namespace ctfp
 
@@ -76,6 +77,7 @@ struct ItemDesc {
     cudaTextureObject_t xtex[kMaxM];   // the axis sampler's x- and y-layered copies (TRILINEAR, TEXEMU)
     cudaTextureObject_t ytex[kMaxM];
     cudaTextureObject_t tex[kMaxM];    // 3D textures (TEXTURE: the reference's own sampler)
+    const float* cvol; // the axis sampler's column copy (four materials)
     const float* mu;   // [E][M]
     const float* W;    // energy weights (weight_index)
     int M, E, interp;
@@ -170,8 +172,7 @@ __device__ __forceinline__ void batch_march(const ItemDesc& it, const ItemTex<M>
     if (AXIS && MODE != INTERP_TEXTURE) {
         const OccView none{nullptr, 0, 0, 0, 0, 0, 0};
         constexpr int AM = MODE == INTERP_TEXTURE ? INTERP_TEXEMU : MODE;  // (not instantiated for TEXTURE)
-        if (axis_is_x(it.g, p)) march_ray_axis<M, AM, 0, false>(it.g, tx.x, tx.y, none, p, v, u, L);
-        else march_ray_axis<M, AM, 1, false>(it.g, tx.x, tx.y, none, p, v, u, L);
+        march_axis<M, AM, false>(it.g, tx.x, tx.y, it.cvol, none, p, v, u, L);
         return;
     }
     const RaySeg s = ray_segment(it.g, p, v, u);
@@ -273,7 +274,7 @@ __device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M
 template <bool ADJOINT, int M, int MODE, bool AXIS>
 struct BatchBudget {
     static constexpr int minb = MODE == INTERP_TRILINEAR
-                                    ? (ADJOINT ? (M <= 2 ? 14 : 12) : 8)
+                                    ? (ADJOINT ? (M <= 2 ? 14 : 12) : (uses_columns(M) && AXIS ? 6 : 8))
                                     : (ADJOINT ? (M <= 2 ? 10 : 8) : (M <= 2 ? 6 : 5));
 };
 
@@ -647,6 +648,7 @@ ctfp_status fill_items(ctfp_batch* b, int kind)
         it.M = M;
         it.E = plan_energies(p);
         it.interp = interp;
+        it.cvol = plan_cvol(p);
         it.mu = plan_mu(p);
         it.W = plan_W(p);
         for (int m = 0; m < it.M; m++) {

@@ -1,6 +1,7 @@
-// ctfp_column.cuh — the adjoint's scatter (SAMPLER_AXIS's march transposed)
-// into z-fastest accumulators, shared by the plan kernel (k_backward) and the
-// batched persistent kernels.
+// ctfp_column.cuh — the z-fastest layout of the volumes' voxels: the four-material
+// march of the axis sampler, and the adjoint's scatter (that sampler's march
+// transposed) into accumulators; shared by the plan kernels and the batched
+// persistent kernels.
 #pragma once
 
 #include <cmath>
@@ -10,12 +11,13 @@
 
 namespace ctfp {
 
-// The accumulators: voxel (x, y, z) is element ((x + 2) * ny' + (y + 2)) * nz' +
+// The layout: voxel (x, y, z) is element ((x + 2) * ny' + (y + 2)) * nz' +
 // (z + 2), ny' = ny + 4, nz' = nz + 4.  Two border voxels surround the volume on
 // every side, so a footprint with its base in [-2, n] on each axis lies in
-// bounds with no test; what falls into the border is never read.  One set
-// serves the views marched along x and those marched along y, and with lanes
-// down the detector's rows (z) a warp's reductions are runs of memory.
+// bounds with no test: the march reads the border as zeros, what the adjoint
+// adds there is never read.  One array serves the views marched along x and
+// those marched along y, and with lanes down the detector's rows (z) a warp's
+// loads and reductions are runs of memory.
 constexpr int kColPad = 2;
 struct ColumnDims {
     unsigned sx, sy, origin;  // element strides of x and y; element of voxel (0, 0, 0)
@@ -36,7 +38,7 @@ __host__ __device__ __forceinline__ bool column_fits(int nx, int ny, int nz)
 {
     return (double)(nx + 2 * kColPad) * (ny + 2 * kColPad) * (nz + 2 * kColPad) < 4294967040.0;
 }
-// 32 x 32 (x, z) tiles of every y: how the gradients are folded; block k's tile.
+// 32 x 32 (x, z) tiles of every y: how the copy is filled and the gradients folded; block k's tile.
 __host__ __device__ __forceinline__ long long column_tiles(int nx, int ny, int nz)
 {
     return (long long)((nx + 31) / 32) * ((nz + 31) / 32) * ny;
@@ -99,6 +101,127 @@ __device__ __forceinline__ RaySeg column_segment(const GeomParams& g, int p, int
     clip_tight(s.az, s.bz, -1.0 - slack, (double)g.nz + slack, s.i0, s.i1);
     if (s.i1 < s.i0) s.i1 = s.i0;
     return s;
+}
+
+// Whether the axis sampler marches M materials over the column copy: 16-byte
+// elements of the four materials side by side, instead of two layered texture
+// copies of each.  A footprint's voxel is then one load for all materials,
+// where the gathers cost the texture unit their time once per material: 48
+// views of 512^3, 218 -> 145 ms (texture returns 90 % busy before).  For fewer
+// materials the loads' lines cost the L1 as much as the gathers: 256^3, 90
+// views, 2 materials 11.9 against 12.1 ms, 3 materials 13.5 against 11.5.
+__host__ __device__ constexpr bool uses_columns(int M) { return M == 4; }
+
+// L_m of one ray over the column copy (or of its part-th of parts equal runs of
+// samples): march_ray_axis with each slot's four corners held for all
+// materials, loaded when the slot's layer or in-layer base changes.
+template <int M, int MODE, bool SKIP>
+__device__ __forceinline__ void march_ray_columns(const GeomParams& g, const float* __restrict__ cvol, const OccView& occ,
+                                                  int p, int v, int u, float* L, int part = 0, int parts = 1)
+{
+    static_assert(M == 4, "elements of four floats");
+    constexpr bool tri = MODE == INTERP_TRILINEAR;
+    RaySeg s = column_segment(g, p, v, u, tri ? 0.0 : 0.5);
+    if (parts > 1) {
+        const int len = (s.i1 - s.i0 + parts - 1) / parts;
+        s.i0 += part * len;
+        s.i1 = min(s.i1, s.i0 + len);
+    }
+    RayRef32 r;
+    if (!tri) r = ray_ref32(g, p, v, u);
+    const ColumnDims cd = column_dims(g.nx, g.ny, g.nz);
+    const bool xl = axis_is_x(g, p);
+    const double bl = xl ? s.bx : s.by, ba = xl ? s.by : s.bx, bz = s.bz, i0 = (double)s.i0;
+    double cl = fma(i0, bl, xl ? s.ax : s.ay), ca = fma(i0, ba, xl ? s.ay : s.ax), cz = fma(i0, bz, s.az);
+    const unsigned sL = xl ? cd.sx : cd.sy, sA = xl ? cd.sy : cd.sx;
+    const float4* const vol = (const float4*)cvol;
+    float4 q0[4], q1[4];  // slots of the even and the odd layer: (a, b), (a + 1, b), (a, b + 1), (a + 1, b + 1)
+#pragma unroll
+    for (int j = 0; j < 4; j++) q0[j] = q1[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    float acc[M] = {0.f, 0.f, 0.f, 0.f}, cmp[M] = {0.f, 0.f, 0.f, 0.f};
+    unsigned h0 = 0xffffffffu, h1 = 0xffffffffu;
+    const auto fetch = [&](unsigned at, float4* q) {
+        const float4 *c0 = vol + at, *c1 = vol + (at + sA);
+        q[0] = __ldg(c0);
+        q[2] = __ldg(c0 + 1);
+        q[1] = __ldg(c1);
+        q[3] = __ldg(c1 + 1);
+    };
+    constexpr int kBlock = 16;
+    for (int ib = s.i0; ib < s.i1; ib += kBlock) {
+        const int ie = min(ib + kBlock, s.i1);
+        float blk[M] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+        for (int i = ib; i < ie; i++) {
+            unsigned lo;
+            bool odd;
+            float g0[4], g1[4];  // the corners' weights of the lower and the upper layer
+            if (tri) {
+                float wl, ul, wa, ua, wz, uz;
+                const int il = axis_weights(cl, wl, ul), ia = axis_weights(ca, wa, ua), iz = axis_weights(cz, wz, uz);
+                cl += bl;
+                ca += ba;
+                cz += bz;
+                if (SKIP) {
+                    Corner c = {};
+                    c.ix = xl ? il : ia;
+                    c.iy = xl ? ia : il;
+                    c.iz = iz;
+                    if (!occ.occupied(c)) continue;
+                }
+                lo = (unsigned)il * sL + ((unsigned)ia * sA + (unsigned)(iz + (int)cd.origin));
+                odd = il & 1;
+                const float w[4] = {ua * uz, wa * uz, ua * wz, wa * wz};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    g0[j] = w[j] * ul;
+                    g1[j] = w[j] * wl;
+                }
+            } else {
+                const Corner c = corner_tex(ref32_coords(g, r, i));
+                if (SKIP && !occ.occupied(c)) continue;
+                // an FP32 coordinate may lie outside the border of the FP64 clip
+                const int x = __vimin_s32_relu(c.ix + kColPad, g.nx + kColPad);
+                const int y = __vimin_s32_relu(c.iy + kColPad, g.ny + kColPad);
+                const int z = __vimin_s32_relu(c.iz + kColPad, g.nz + kColPad);
+                lo = (unsigned)x * cd.sx + (unsigned)y * cd.sy + (unsigned)z;
+                odd = (xl ? x : y) & 1;
+                float w[8];
+                texunit_weights(c.qx, c.qy, c.qz, w);
+                g0[0] = w[0]; g0[2] = w[4]; g1[1] = w[3]; g1[3] = w[7];
+                g0[1] = xl ? w[2] : w[1]; g0[3] = xl ? w[6] : w[5];
+                g1[0] = xl ? w[1] : w[2]; g1[2] = xl ? w[5] : w[6];
+            }
+            const unsigned hi = lo + sL, f0 = odd ? hi : lo, f1 = odd ? lo : hi;
+            if (f0 != h0) fetch(f0, q0);
+            if (f1 != h1) fetch(f1, q1);
+            h0 = f0;
+            h1 = f1;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float a = odd ? g1[j] : g0[j], b = odd ? g0[j] : g1[j];
+                blk[0] = fmaf(q1[j].x, b, fmaf(q0[j].x, a, blk[0]));
+                blk[1] = fmaf(q1[j].y, b, fmaf(q0[j].y, a, blk[1]));
+                blk[2] = fmaf(q1[j].z, b, fmaf(q0[j].z, a, blk[2]));
+                blk[3] = fmaf(q1[j].w, b, fmaf(q0[j].w, a, blk[3]));
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < M; m++) kahan_add(acc[m], cmp[m], blk[m]);
+    }
+#pragma unroll
+    for (int m = 0; m < M; m++) L[m] = g.dx * (acc[m] - cmp[m]);
+}
+
+// L_m of one ray of the axis sampler, over whichever copies M materials use.
+template <int M, int MODE, bool SKIP>
+__device__ __forceinline__ void march_axis(const GeomParams& g, const cudaTextureObject_t* xtex,
+                                           const cudaTextureObject_t* ytex, const float* cvol, const OccView& occ, int p,
+                                           int v, int u, float* L, int part = 0, int parts = 1)
+{
+    if constexpr (uses_columns(M)) march_ray_columns<M, MODE, SKIP>(g, cvol, occ, p, v, u, L, part, parts);
+    else if (axis_is_x(g, p)) march_ray_axis<M, MODE, 0, SKIP>(g, xtex, ytex, occ, p, v, u, L, part, parts);
+    else march_ray_axis<M, MODE, 1, SKIP>(g, xtex, ytex, occ, p, v, u, L, part, parts);
 }
 
 // ---------------------------------------------------------------------------

@@ -25,6 +25,10 @@ namespace ctfp {
 
 namespace {
 
+struct VolPtrs {
+    const float* p[kMaxM];
+};
+
 template <int M, int SAMPLER>
 __device__ __forceinline__ void load_corners(const MarchParams& prm, const Corner& c, float (*v)[8])
 {
@@ -181,8 +185,7 @@ __global__ void __launch_bounds__(256, MINB) k_forward_axis(const MarchParams pr
         if (p >= pend) break;
         float L[M];
         const OccView ov{prm.occ, prm.occ_x, prm.occ_y, prm.g.nx, prm.g.ny, prm.g.nz, kOccShift};
-        if (axis_is_x(prm.g, p)) march_ray_axis<M, MODE, 0, SKIP>(prm.g, prm.xtex, prm.ytex, ov, p, v, u, L);
-        else march_ray_axis<M, MODE, 1, SKIP>(prm.g, prm.xtex, prm.ytex, ov, p, v, u, L);
+        march_axis<M, MODE, SKIP>(prm.g, prm.xtex, prm.ytex, prm.cvol, ov, p, v, u, L);
         const int64_t ray = (int64_t)(p - prm.out_view0) * npix + pix;
         if (prm.L) store_L<M>(prm.L, ray, L);
         if (SPECTRAL) {
@@ -202,7 +205,7 @@ __global__ void __launch_bounds__(256, MINB) k_forward_axis(const MarchParams pr
 // The energies' partial sums are spectral()'s four accumulators, combined in
 // its order, so I and IAbs equal its values for the same L.
 template <int M, int MODE, bool SKIP, bool SPECTRAL>
-__global__ void __launch_bounds__(128, 8) k_forward_axis_split(const MarchParams prm, int shift)
+__global__ void __launch_bounds__(128, uses_columns(M) ? 6 : 8) k_forward_axis_split(const MarchParams prm, int shift)
 {
     extern __shared__ __align__(16) float s_mu[];
     if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E, M);
@@ -218,8 +221,7 @@ __global__ void __launch_bounds__(128, 8) k_forward_axis_split(const MarchParams
     for (int m = 0; m < M; m++) L[m] = 0.f;
     if (on) {
         const OccView ov{prm.occ, prm.occ_x, prm.occ_y, prm.g.nx, prm.g.ny, prm.g.nz, kOccShift};
-        if (axis_is_x(prm.g, p)) march_ray_axis<M, MODE, 0, SKIP>(prm.g, prm.xtex, prm.ytex, ov, p, v, u, L, part, 1 << shift);
-        else march_ray_axis<M, MODE, 1, SKIP>(prm.g, prm.xtex, prm.ytex, ov, p, v, u, L, part, 1 << shift);
+        march_axis<M, MODE, SKIP>(prm.g, prm.xtex, prm.ytex, prm.cvol, ov, p, v, u, L, part, 1 << shift);
     }
     for (int d = rows; d < 32; d <<= 1)
 #pragma unroll
@@ -313,6 +315,32 @@ __global__ void __launch_bounds__(256) k_axis_fill(const float* __restrict__ vol
             const int y = y0 + tx, x = x0 + ty;  // x-layered: layer x, texel (y, z)
             if (x < nx && y < ny) surf2DLayeredwrite(t[tx][ty], xs, y * (int)sizeof(float), z, x + 1);
         }
+    }
+}
+
+// The column copy's interior: for one y, a 32 x 32 (x, z) tile of the four
+// materials through shared memory, read along x and written along z as 16-byte
+// elements.  Block (32, 8); one block per tile, column_tile.
+__global__ void __launch_bounds__(256) k_column_fill(const VolPtrs vol, int nx, int ny, int nz, float* __restrict__ cvol)
+{
+    __shared__ float t[4][32][33];
+    int x0, y, z0;
+    column_tile(blockIdx.x, nx, nz, x0, y, z0);
+    const int tx = threadIdx.x;
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int x = x0 + tx, z = z0 + k;
+        if (x < nx && z < nz) {
+#pragma unroll
+            for (int m = 0; m < 4; m++) t[m][k][tx] = __ldg(vol.p[m] + ((size_t)z * ny + y) * nx + x);
+        }
+    }
+    __syncthreads();
+    const ColumnDims cd = column_dims(nx, ny, nz);
+    for (int k = threadIdx.y; k < 32; k += 8) {
+        const int x = x0 + k, z = z0 + tx;
+        if (x < nx && z < nz)
+            ((float4*)cvol)[(size_t)x * cd.sx + (size_t)y * cd.sy + (size_t)z + cd.origin] =
+                make_float4(t[0][tx][k], t[1][tx][k], t[2][tx][k], t[3][tx][k]);
     }
 }
 
@@ -1264,6 +1292,18 @@ cudaError_t launch_axis_fill(const float* vol, int nx, int ny, int nz, cudaSurfa
     return cudaGetLastError();
 }
 
+bool axis_uses_columns(int M) { return uses_columns(M); }
+
+size_t column_floats(int nx, int ny, int nz) { return column_dims(nx, ny, nz).elems * 4; }
+
+cudaError_t launch_column_fill(const float* const* vol, int nx, int ny, int nz, float* cvol, cudaStream_t st)
+{
+    VolPtrs vp = {};
+    for (int m = 0; m < kMaxM; m++) vp.p[m] = vol[m];
+    k_column_fill<<<(unsigned)column_tiles(nx, ny, nz), dim3(32, 8), 0, st>>>(vp, nx, ny, nz, cvol);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_spectral_from_L(const MarchParams& prm, int M, cudaStream_t st)
 {
     const dim3 block(256, 1);
@@ -1395,10 +1435,6 @@ namespace {
 // One thread per voxel: a non-zero voxel marks every brick whose dilated
 // range [8b - 1, 8b + 7] holds it (b = (x + 1) >> 3, and b - 1 when x + 1 is a
 // multiple of 8), per axis.  Concurrent stores all write 1.
-struct VolPtrs {
-    const float* p[kMaxM];
-};
-
 __global__ void k_occupancy(const VolPtrs vol, int M, int nx, int ny, int nz, int ox, int oy, uint8_t* occ)
 {
     const int64_t n = (int64_t)nx * ny * nz;

@@ -13,6 +13,7 @@ struct MarchParams {
     cudaTextureObject_t ltex[kMaxM];  // same volumes as layered 2D textures (SAMPLER_LAYERED)
     cudaTextureObject_t xtex[kMaxM];  // SAMPLER_AXIS: layered along x (layer x, texel (y, z))
     cudaTextureObject_t ytex[kMaxM];  // SAMPLER_AXIS: layered along y (layer y, texel (x, z))
+    const float* cvol;                // SAMPLER_AXIS, four materials: the column copy instead (ctfp_column.cuh)
     float* L;                         // [P][V][U][M] path integrals (out, may be null)
     const float* Lin;                 // [P][V][U][M] path integrals (in, epilogue/adjoint)
     float* I;                         // [P][V][U] (may be null)
@@ -81,7 +82,12 @@ cudaError_t launch_count_support(const GeomParams& g, unsigned long long* out, c
 // of views view0.. (interp selects exact or texture-unit bilinear weights).
 cudaError_t launch_shift_views(const float* in, float* out, const GeomParams& g, int M, int interp, int view0,
                                int n_views, cudaStream_t st);
-// SAMPLER_AXIS: writes one volume [nz][ny][nx] into its x-layered copy
+// SAMPLER_AXIS: whether M materials use the column copy, its floats, and its
+// interior from the volumes (the border stays as allocated: zero).
+bool axis_uses_columns(int M);
+size_t column_floats(int nx, int ny, int nz);
+cudaError_t launch_column_fill(const float* const* vol, int nx, int ny, int nz, float* cvol, cudaStream_t st);
+// Otherwise: writes one volume [nz][ny][nx] into its x-layered copy
 // (surface xs: texture layer x + 1, texel (y, z)) and its y-layered copy (ys:
 // texture layer y + 1, texel (x, z)).
 cudaError_t launch_axis_fill(const float* vol, int nx, int ny, int nz, cudaSurfaceObject_t xs, cudaSurfaceObject_t ys,
