@@ -313,9 +313,13 @@ ctfp_status upload_textures(ctfp_plan* p, const float* const* volumes, cudaStrea
         return CTFP_OK;
     }
     if (uses_axis(p)) {
-        for (int m = 0; m < p->M; m++)
-            CTFP_CUDA(launch_axis_fill(volumes[m], (int)p->geom.pNumX, (int)p->geom.pNumY, (int)p->geom.pNumZ,
-                                       p->xsurf[m], p->ysurf[m], st));
+        AxisCopies c = {};
+        for (int m = 0; m < p->M; m++) {
+            c.vol[m] = volumes[m];
+            c.xs[m] = p->xsurf[m];
+            c.ys[m] = p->ysurf[m];
+        }
+        CTFP_CUDA(launch_axis_fill(c, p->M, (int)p->geom.pNumX, (int)p->geom.pNumY, (int)p->geom.pNumZ, st));
         return CTFP_OK;
     }
     if (!tex3d && !uses_layered(p)) return CTFP_OK;

@@ -294,12 +294,15 @@ __global__ void __launch_bounds__(256) k_axis_gather_count(const GeomParams g, i
 // of one z slice in shared memory so that both copies are written along their
 // texel rows; voxel layer l is texture layer l + 1 (layer 0 and the last
 // layer are zeros, k_axis_zero_layers).  Block (32, 8); grid (ceil(nx / 32),
-// ceil(ny / 32), nz).
-__global__ void __launch_bounds__(256) k_axis_fill(const float* __restrict__ vol, int nx, int ny,
-                                                   cudaSurfaceObject_t xs, cudaSurfaceObject_t ys)
+// ceil(ny / 32), nz * materials): one launch for all of them (two launches of
+// 5 us were a third of the smallest forward).
+__global__ void __launch_bounds__(256) k_axis_fill(const AxisCopies c, int nx, int ny, int nz)
 {
     __shared__ float t[32][33];
-    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, z = blockIdx.z;
+    const int m = blockIdx.z / nz, z = blockIdx.z - m * nz;
+    const float* __restrict__ vol = c.vol[m];
+    const cudaSurfaceObject_t xs = c.xs[m], ys = c.ys[m];
+    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
     const int tx = threadIdx.x;
     for (int ty = threadIdx.y; ty < 32; ty += 8) {
         const int x = x0 + tx, y = y0 + ty;
@@ -1283,13 +1286,23 @@ cudaError_t launch_axis_zero_pads(int nx, int ny, int nz, cudaSurfaceObject_t xs
     return cudaGetLastError();
 }
 
-cudaError_t launch_axis_fill(const float* vol, int nx, int ny, int nz, cudaSurfaceObject_t xs, cudaSurfaceObject_t ys,
-                             cudaStream_t st)
+cudaError_t launch_axis_fill(const AxisCopies& copies, int M, int nx, int ny, int nz, cudaStream_t st)
 {
-    const dim3 grid((nx + 31) / 32, (ny + 31) / 32, nz);
-    if (grid.x == 0 || grid.y == 0 || grid.z == 0) return cudaSuccess;
-    k_axis_fill<<<grid, dim3(32, 8), 0, st>>>(vol, nx, ny, xs, ys);
-    return cudaGetLastError();
+    // grid.z holds at most 65535 slices
+    const int per = std::max(1, std::min(M, 65535 / nz));
+    for (int m = 0; m < M; m += per) {
+        const int n = std::min(per, M - m);
+        AxisCopies c = copies;
+        for (int k = 0; k < n; k++) {
+            c.vol[k] = copies.vol[m + k];
+            c.xs[k] = copies.xs[m + k];
+            c.ys[k] = copies.ys[m + k];
+        }
+        k_axis_fill<<<dim3((nx + 31) / 32, (ny + 31) / 32, nz * n), dim3(32, 8), 0, st>>>(c, nx, ny, nz);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 bool axis_uses_columns(int M) { return uses_columns(M); }

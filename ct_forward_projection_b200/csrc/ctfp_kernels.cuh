@@ -87,11 +87,14 @@ cudaError_t launch_shift_views(const float* in, float* out, const GeomParams& g,
 bool axis_uses_columns(int M);
 size_t column_floats(int nx, int ny, int nz);
 cudaError_t launch_column_fill(const float* const* vol, int nx, int ny, int nz, float* cvol, cudaStream_t st);
-// Otherwise: writes one volume [nz][ny][nx] into its x-layered copy
-// (surface xs: texture layer x + 1, texel (y, z)) and its y-layered copy (ys:
-// texture layer y + 1, texel (x, z)).
-cudaError_t launch_axis_fill(const float* vol, int nx, int ny, int nz, cudaSurfaceObject_t xs, cudaSurfaceObject_t ys,
-                             cudaStream_t st);
+// Otherwise: writes each volume [nz][ny][nx] into its x-layered copy (surface
+// xs: texture layer x + 1, texel (y, z)) and its y-layered copy (ys: texture
+// layer y + 1, texel (x, z)).
+struct AxisCopies {
+    const float* vol[kMaxM];
+    cudaSurfaceObject_t xs[kMaxM], ys[kMaxM];
+};
+cudaError_t launch_axis_fill(const AxisCopies& copies, int M, int nx, int ny, int nz, cudaStream_t st);
 // The axis march's texture quad-gathers over every view of a problem, with the
 // launch shape's tile and lane layout: out[0] += quads, out[1] += samples.
 cudaError_t launch_axis_gather_count(const GeomParams& g, int interp, const LaunchShape& ls, unsigned long long* out,
