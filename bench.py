@@ -617,6 +617,8 @@ def texture_roof(pr, interp, sampler, local, cache):
     voxel-sample (ctfp_sampler_peak tex3d).  cache holds the probe results."""
     from ct_forward_projection_b200.projector import sampler_peak
     kind = "tex3d" if interp == "texture" else ("layered" if sampler in ("layered", "axis") else None)
+    if kind == "layered" and sampler == "axis" and pr.M == 4:
+        return None, None  # four materials march the column copy: loads, no texture gathers
     if kind is None:
         return None, None
     if kind not in cache:

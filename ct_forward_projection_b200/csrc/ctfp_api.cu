@@ -61,7 +61,7 @@ struct ctfp_plan {
     size_t fs_raw_elems = 0;
     float* d_fs_L = nullptr;
     size_t fs_L_elems = 0;
-    float* d_gcol = nullptr;  // adjoint accumulators (grown on demand)
+    float* d_gcol = nullptr;  // adjoint accumulators (allocated on first backward)
     size_t gcol_elems = 0;
     // staging for ctfp_forward_host
     float* h2d_vol[kMaxM] = {};
@@ -422,7 +422,9 @@ ctfp_status scatter_and_fold(ctfp_plan* p, MarchParams prm, bool from_gL, cudaSt
     if (accum_fits(p->gp.nx, p->gp.ny, p->gp.nz)) {  // else prm.gcol stays null: no accumulators
         prm.sets = accum_set_count(p->gp, prm.n_views, p->M);
         prm.set_floats = accum_floats(p->gp.nx, p->gp.ny, p->gp.nz, p->M);
-        const ctfp_status st = ensure_scratch(p->d_gcol, p->gcol_elems, prm.set_floats * prm.sets);
+        // sized once, for a call over every view
+        const size_t most = prm.set_floats * accum_set_count(p->gp, p->gp.P, p->M);
+        const ctfp_status st = ensure_scratch(p->d_gcol, p->gcol_elems, most);
         if (st != CTFP_OK) return st;
         prm.gcol = p->d_gcol;
         CTFP_CUDA(cudaMemsetAsync(prm.gcol, 0, sizeof(float) * prm.set_floats * prm.sets, s));

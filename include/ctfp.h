@@ -103,7 +103,10 @@ typedef enum ctfp_sampler {
      * their 2x2 in-layer footprint or move it one layer on; the gathers a ray
      * already holds are kept in registers and only the missing layers are
      * fetched.  Results agree with the layered sampler to FP32 rounding (the
-     * layer axis is interpolated last).  The default; needs pNumX, pNumY <= 2046
+     * layer axis is interpolated last).  Plans of four materials hold one
+     * z-fastest copy instead, the four materials of a voxel side by side, and
+     * load the missing corners from it; plans of at most 700 000 rays march a
+     * ray with 2, 4 or 8 threads.  The default; needs pNumX, pNumY <= 2046
      * and pNumZ <= 32768 (else the layered sampler, else the global one). */
     CTFP_SAMPLER_AXIS = 4
 } ctfp_sampler;
@@ -503,7 +506,9 @@ ctfp_status ctfp_count_support_samples(ctfp_plan* plan, int64_t* out);
  * (as the layered sampler's two gathers do) gives 0.5 (16 quads per 32
  * samples), so the axis march's texture roof is ctfp_sampler_peak
  * (CTFP_SAMPLER_LAYERED) x 0.5 / quad_gathers_per_sample voxel-samples/s.
- * Does not depend on the volumes.  No counterpart in the reference. */
+ * Does not depend on the volumes.  (A plan of four materials loads its corners
+ * without the texture unit; the count is then that of the same reuse by
+ * gathers.)  No counterpart in the reference. */
 ctfp_status ctfp_axis_gather_count(ctfp_plan* plan, double* quad_gathers_per_sample);
 
 /* Message of the last error on the calling thread ("" if none). */
