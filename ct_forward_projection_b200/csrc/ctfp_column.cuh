@@ -99,6 +99,18 @@ __device__ __forceinline__ RaySeg column_segment(const GeomParams& g, int p, int
     clip_tight(s.ax, s.bx, -1.0 - slack, (double)g.nx + slack, s.i0, s.i1);
     clip_tight(s.ay, s.by, -1.0 - slack, (double)g.ny + slack, s.i0, s.i1);
     clip_tight(s.az, s.bz, -1.0 - slack, (double)g.nz + slack, s.i0, s.i1);
+    // The coordinates are linear in i, so the first and the last sample within
+    // the border mean that all are.  Where 1e-6 of a sample is no longer a
+    // fraction of a voxel (voxels a millionth of the step flat), or a coordinate
+    // is no number, the clip alone does not place them there.
+    const auto inside = [&](int i) {
+        const double t = (double)i;
+        const double x = fma(t, s.bx, s.ax), y = fma(t, s.by, s.ay), z = fma(t, s.bz, s.az);
+        return x > -1.75 && y > -1.75 && z > -1.75 && x < (double)g.nx + 0.75 && y < (double)g.ny + 0.75 &&
+               z < (double)g.nz + 0.75;
+    };
+    while (s.i0 < s.i1 && !inside(s.i0)) s.i0++;
+    while (s.i0 < s.i1 && !inside(s.i1 - 1)) s.i1--;
     if (s.i1 < s.i0) s.i1 = s.i0;
     return s;
 }
