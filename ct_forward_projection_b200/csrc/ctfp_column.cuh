@@ -68,8 +68,11 @@ __device__ __forceinline__ void clip_tight(double a, double b, double lo, double
 
 // ray_segment's coordinates with one reciprocal of R and the plan's
 // reciprocals of the voxel sizes (each within 2^-52 relative of the quotient:
-// 1e-13 voxel), clipped by clip_tight to (-1 - slack, n + slack).
-__device__ __forceinline__ RaySeg column_segment(const GeomParams& g, int p, int v, int u, double slack)
+// 1e-13 voxel), clipped by clip_tight.  For the exact coordinates only: the
+// texture emulation's FP32 ones may lie voxels away from these, so there
+// ray_segment's samples count, as in every other sampler, and each footprint
+// is moved to the border where it lies beyond it.
+__device__ __forceinline__ RaySeg column_segment(const GeomParams& g, int p, int v, int u)
 {
     const double dsz = g.dSize, sdd = g.sdd, sod = g.sod;
     const double detU = (double)g.dHalfLU - dsz / 2 - (double)u * dsz;
@@ -96,9 +99,9 @@ __device__ __forceinline__ RaySeg column_segment(const GeomParams& g, int p, int
     s.az = (kw * t0 + cw) * g.qz; s.bz = kw * dt * g.qz;
     s.i0 = 0;
     s.i1 = g.K;
-    clip_tight(s.ax, s.bx, -1.0 - slack, (double)g.nx + slack, s.i0, s.i1);
-    clip_tight(s.ay, s.by, -1.0 - slack, (double)g.ny + slack, s.i0, s.i1);
-    clip_tight(s.az, s.bz, -1.0 - slack, (double)g.nz + slack, s.i0, s.i1);
+    clip_tight(s.ax, s.bx, -1.0, (double)g.nx, s.i0, s.i1);
+    clip_tight(s.ay, s.by, -1.0, (double)g.ny, s.i0, s.i1);
+    clip_tight(s.az, s.bz, -1.0, (double)g.nz, s.i0, s.i1);
     // The coordinates are linear in i, so the first and the last sample within
     // the border mean that all are.  Where 1e-6 of a sample is no longer a
     // fraction of a voxel (voxels a millionth of the step flat), or a coordinate
@@ -133,7 +136,7 @@ __device__ __forceinline__ void march_ray_columns(const GeomParams& g, const flo
 {
     static_assert(M == 4, "elements of four floats");
     constexpr bool tri = MODE == INTERP_TRILINEAR;
-    RaySeg s = column_segment(g, p, v, u, tri ? 0.0 : 0.5);
+    RaySeg s = tri ? column_segment(g, p, v, u) : ray_segment(g, p, v, u);
     if (parts > 1) {
         const int len = (s.i1 - s.i0 + parts - 1) / parts;
         s.i0 += part * len;
@@ -192,7 +195,7 @@ __device__ __forceinline__ void march_ray_columns(const GeomParams& g, const flo
             } else {
                 const Corner c = corner_tex(ref32_coords(g, r, i));
                 if (SKIP && !occ.occupied(c)) continue;
-                // an FP32 coordinate may lie outside the border of the FP64 clip
+                // an FP32 coordinate may lie outside the border
                 const int x = __vimin_s32_relu(c.ix + kColPad, g.nx + kColPad);
                 const int y = __vimin_s32_relu(c.iy + kColPad, g.ny + kColPad);
                 const int z = __vimin_s32_relu(c.iz + kColPad, g.nz + kColPad);
@@ -399,7 +402,7 @@ template <int M, bool MERGE>
 __device__ __forceinline__ void scatter_trilinear(const GeomParams& gp, float* acc, bool on, int p, int v, int u,
                                                   const float* g)
 {
-    RaySeg s = column_segment(gp, p, v, u, 0.0);
+    RaySeg s = column_segment(gp, p, v, u);
     const ColumnDims cd = column_dims(gp.nx, gp.ny, gp.nz);
     const bool xl = axis_is_x(gp, p);
     const double bl = xl ? s.bx : s.by, ba = xl ? s.by : s.bx, bz = s.bz;
@@ -436,7 +439,7 @@ template <int M, bool MERGE, bool XL>
 __device__ __forceinline__ void scatter_texemu(const GeomParams& gp, float* acc, bool on, int p, int v, int u,
                                                const float* g)
 {
-    const RaySeg s = column_segment(gp, p, v, u, 0.5);
+    const RaySeg s = ray_segment(gp, p, v, u);
     const RayRef32 r = ray_ref32(gp, p, v, u);
     const ColumnDims cd = column_dims(gp.nx, gp.ny, gp.nz);
     const unsigned sL = XL ? cd.sx : cd.sy, sA = XL ? cd.sy : cd.sx;
