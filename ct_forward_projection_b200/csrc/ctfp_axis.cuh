@@ -81,7 +81,8 @@ __device__ __forceinline__ Corner axis_corner(const GeomParams& g, const RayRef3
     return corner_tex(ref32_coords(g, r, i));
 }
 
-// L_m for one ray with the axis sampler (AX 0: layered along x, 1: along y).
+// The sums over one ray's samples with the axis sampler (AX 0: layered along x,
+// 1: along y), as Kahan pairs: sum m is acc[m] - cmp[m].
 // Each ray is marched on its own (from its own first sample), so its result
 // does not depend on the launch shape.  (Stepping a warp's lanes through
 // common sample indices instead, from the earliest entry to the latest exit
@@ -91,7 +92,7 @@ __device__ __forceinline__ Corner axis_corner(const GeomParams& g, const RayRef3
 template <int M, int MODE, int AX, bool SKIP>
 __device__ __forceinline__ void march_ray_axis(const GeomParams& g, const cudaTextureObject_t* xtex,
                                                const cudaTextureObject_t* ytex, const OccView& occ, int p, int v,
-                                               int u, float* L, int part = 0, int parts = 1)
+                                               int u, float* acc, float* cmp, int part, int parts)
 {
     RaySeg s = ray_segment(g, p, v, u);
     if (parts > 1) {
@@ -102,7 +103,6 @@ __device__ __forceinline__ void march_ray_axis(const GeomParams& g, const cudaTe
     RayRef32 r;
     if (MODE != INTERP_TRILINEAR) r = ray_ref32(g, p, v, u);
     const cudaTextureObject_t* tx = AX == 0 ? xtex : ytex;
-    float acc[M], cmp[M];
     float4 q0[M], q1[M];  // slot 0: the even layer of the pair, slot 1: the odd one
 #pragma unroll
     for (int m = 0; m < M; m++) {
@@ -189,8 +189,6 @@ __device__ __forceinline__ void march_ray_axis(const GeomParams& g, const cudaTe
 #pragma unroll
     for (int m = 0; m < M; m++) kahan_add(acc[m], cmp[m], blk[m]);
     }
-#pragma unroll
-    for (int m = 0; m < M; m++) L[m] = g.dx * (acc[m] - cmp[m]);
 }
 
 // The gathers the axis march of one ray issues, as the texture unit sees

@@ -127,12 +127,12 @@ __device__ __forceinline__ RaySeg column_segment(const GeomParams& g, int p, int
 // views, 2 materials 11.9 against 12.1 ms, 3 materials 13.5 against 11.5.
 __host__ __device__ constexpr bool uses_columns(int M) { return M == 4; }
 
-// L_m of one ray over the column copy (or of its part-th of parts equal runs of
-// samples): march_ray_axis with each slot's four corners held for all
+// The sums of one ray over the column copy (or of its part-th of parts equal runs
+// of samples): march_ray_axis with each slot's four corners held for all
 // materials, loaded when the slot's layer or in-layer base changes.
 template <int M, int MODE, bool SKIP>
 __device__ __forceinline__ void march_ray_columns(const GeomParams& g, const float* __restrict__ cvol, const OccView& occ,
-                                                  int p, int v, int u, float* L, int part = 0, int parts = 1)
+                                                  int p, int v, int u, float* acc, float* cmp, int part, int parts)
 {
     static_assert(M == 4, "elements of four floats");
     constexpr bool tri = MODE == INTERP_TRILINEAR;
@@ -153,7 +153,8 @@ __device__ __forceinline__ void march_ray_columns(const GeomParams& g, const flo
     float4 q0[4], q1[4];  // slots of the even and the odd layer: (a, b), (a + 1, b), (a, b + 1), (a + 1, b + 1)
 #pragma unroll
     for (int j = 0; j < 4; j++) q0[j] = q1[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    float acc[M] = {0.f, 0.f, 0.f, 0.f}, cmp[M] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int m = 0; m < M; m++) acc[m] = cmp[m] = 0.f;
     unsigned h0 = 0xffffffffu, h1 = 0xffffffffu;
     const auto fetch = [&](unsigned at, float4* q) {
         const float4 *c0 = vol + at, *c1 = vol + (at + sA);
@@ -224,19 +225,31 @@ __device__ __forceinline__ void march_ray_columns(const GeomParams& g, const flo
 #pragma unroll
         for (int m = 0; m < M; m++) kahan_add(acc[m], cmp[m], blk[m]);
     }
-#pragma unroll
-    for (int m = 0; m < M; m++) L[m] = g.dx * (acc[m] - cmp[m]);
 }
 
-// L_m of one ray of the axis sampler, over whichever copies M materials use.
+// The sums of one ray of the axis sampler, or of one part of it, over whichever
+// copies M materials use.
+template <int M, int MODE, bool SKIP>
+__device__ __forceinline__ void march_axis_sums(const GeomParams& g, const cudaTextureObject_t* xtex,
+                                                const cudaTextureObject_t* ytex, const float* cvol,
+                                                const OccView& occ, int p, int v, int u, float* acc, float* cmp,
+                                                int part = 0, int parts = 1)
+{
+    if constexpr (uses_columns(M)) march_ray_columns<M, MODE, SKIP>(g, cvol, occ, p, v, u, acc, cmp, part, parts);
+    else if (axis_is_x(g, p)) march_ray_axis<M, MODE, 0, SKIP>(g, xtex, ytex, occ, p, v, u, acc, cmp, part, parts);
+    else march_ray_axis<M, MODE, 1, SKIP>(g, xtex, ytex, occ, p, v, u, acc, cmp, part, parts);
+}
+
+// L_m of one ray.
 template <int M, int MODE, bool SKIP>
 __device__ __forceinline__ void march_axis(const GeomParams& g, const cudaTextureObject_t* xtex,
                                            const cudaTextureObject_t* ytex, const float* cvol, const OccView& occ, int p,
-                                           int v, int u, float* L, int part = 0, int parts = 1)
+                                           int v, int u, float* L)
 {
-    if constexpr (uses_columns(M)) march_ray_columns<M, MODE, SKIP>(g, cvol, occ, p, v, u, L, part, parts);
-    else if (axis_is_x(g, p)) march_ray_axis<M, MODE, 0, SKIP>(g, xtex, ytex, occ, p, v, u, L, part, parts);
-    else march_ray_axis<M, MODE, 1, SKIP>(g, xtex, ytex, occ, p, v, u, L, part, parts);
+    float acc[M], cmp[M];
+    march_axis_sums<M, MODE, SKIP>(g, xtex, ytex, cvol, occ, p, v, u, acc, cmp);
+#pragma unroll
+    for (int m = 0; m < M; m++) L[m] = g.dx * (acc[m] - cmp[m]);
 }
 
 // ---------------------------------------------------------------------------

@@ -477,6 +477,17 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float x)
     s = t;
 }
 
+// The sum of two Kahan pairs (s - c and s2 - c2): what the addition of s and s2
+// rounds off goes into the compensation (Knuth's two-sum, exact), so joining a
+// ray's parts costs no accuracy.  Symmetric in the pairs.
+__device__ __forceinline__ void kahan_join(float& s, float& c, float s2, float c2)
+{
+    const float t = s + s2;
+    const float b = t - s;
+    c = (c + c2) - ((s - (t - b)) + (s2 - b));
+    s = t;
+}
+
 // The energy weights W, laid out for the marches' warps: pixels in blocks of 4
 // columns x 8 rows (lane (v & 7) * 4 + (u & 3)), a block's energies in groups of
 // 4, so that a lane loads 4 energies with one 16-byte load and a warp of 4

@@ -216,16 +216,19 @@ __global__ void __launch_bounds__(128, uses_columns(M) ? 6 : 8) k_forward_axis_s
     const int64_t npix = (int64_t)prm.g.U * prm.g.V;
     const int64_t pix = (int64_t)v * prm.g.U + u;
     const int64_t ray = (int64_t)(p - prm.out_view0) * npix + pix;
-    float L[M];
+    float L[M], cmp[M];  // the sum's Kahan pair, then L
 #pragma unroll
-    for (int m = 0; m < M; m++) L[m] = 0.f;
+    for (int m = 0; m < M; m++) L[m] = cmp[m] = 0.f;
     if (on) {
         const OccView ov{prm.occ, prm.occ_x, prm.occ_y, prm.g.nx, prm.g.ny, prm.g.nz, kOccShift};
-        march_axis<M, MODE, SKIP>(prm.g, prm.xtex, prm.ytex, prm.cvol, ov, p, v, u, L, part, 1 << shift);
+        march_axis_sums<M, MODE, SKIP>(prm.g, prm.xtex, prm.ytex, prm.cvol, ov, p, v, u, L, cmp, part, 1 << shift);
     }
     for (int d = rows; d < 32; d <<= 1)
 #pragma unroll
-        for (int m = 0; m < M; m++) L[m] += __shfl_xor_sync(0xffffffffu, L[m], d);
+        for (int m = 0; m < M; m++)
+            kahan_join(L[m], cmp[m], __shfl_xor_sync(0xffffffffu, L[m], d), __shfl_xor_sync(0xffffffffu, cmp[m], d));
+#pragma unroll
+    for (int m = 0; m < M; m++) L[m] = prm.g.dx * (L[m] - cmp[m]);
     if (on && part == 0 && prm.L) store_L<M>(prm.L, ray, L);
     if (SPECTRAL) {
         // accumulators of this lane: two of the four (2 lanes per ray) or one
