@@ -1,4 +1,4 @@
-"""Rays shared by lanes are summed as accurately as rays marched by one thread:
+"""How accurately a ray is summed.  Rays shared by lanes against rays of one thread:
 the same rays through a plan small enough to share them and through one of 64 or
 16 times the views, both against the FP64 oracle."""
 import numpy as np
@@ -28,3 +28,27 @@ def test_split_sums_as_accurate_as_one_thread(cuda_ok, views, more, M):
     assert on.sum() > 10000
     # either is an estimate from over 10 000 rays, good to about a percent
     assert rms[0] <= 1.05 * rms[1], rms
+
+
+@pytest.mark.parametrize("mode", ["trilinear", "texemu"])
+@pytest.mark.parametrize("views", [4, 64])  # 8 lanes a ray; 4 lanes
+def test_four_materials_as_accurate_as_two(cuda_ok, views, mode):
+    """The column copy's march of four materials against the texture gathers'
+    march of the first two: the same samples, so the same rounding error (texture
+    emulation: against the layered sampler, which compensates every sample)."""
+    d = small_geometry(n=(128, 128, 96), views=views, U=64, V=64, length=128.0, pitch=3.0)
+    vols = random_volumes(d, 4, 12)
+    dev = [torch.from_numpy(v).cuda() for v in vols]
+    got = {}
+    for M in (2, 4):
+        with Projector(d, M, mode) as pr:
+            got[M] = pr.line_integrals(dev[:M])[..., :2].double().cpu().numpy()
+            if mode == "texemu" and M == 2:
+                pr.set_sampler("layered")
+                ref = pr.line_integrals(dev[:M]).double().cpu().numpy()
+    if mode == "trilinear":
+        ref = O.line_integrals(d, vols[:2], O.TRILINEAR).reshape(got[2].shape)
+    on = ref > 0.1 * ref.max()
+    assert on.sum() > 10000
+    rms = {M: float(np.sqrt(np.mean(((g - ref)[on] / ref[on]) ** 2))) for M, g in got.items()}
+    assert rms[4] <= 1.05 * rms[2], rms
