@@ -62,7 +62,7 @@ struct ctfp_plan {
     float* d_fs_L = nullptr;
     size_t fs_L_elems = 0;
     float* d_gcol = nullptr;  // adjoint accumulators (allocated on first backward)
-    size_t gcol_elems = 0;
+    int gcol_sets = 0;  // sets of them
     // staging for ctfp_forward_host
     float* h2d_vol[kMaxM] = {};
     float* d2h_I = nullptr;
@@ -420,12 +420,20 @@ ctfp_status prepare_volumes(ctfp_plan* p, const float* const* volumes, cudaStrea
 ctfp_status scatter_and_fold(ctfp_plan* p, MarchParams prm, bool from_gL, cudaStream_t s)
 {
     if (accum_fits(p->gp.nx, p->gp.ny, p->gp.nz)) {  // else prm.gcol stays null: no accumulators
-        prm.sets = accum_set_count(p->gp, prm.n_views, p->M);
         prm.set_floats = accum_floats(p->gp.nx, p->gp.ny, p->gp.nz, p->M);
-        // sized once, for a call over every view
-        const size_t most = prm.set_floats * accum_set_count(p->gp, p->gp.P, p->M);
-        const ctfp_status st = ensure_scratch(p->d_gcol, p->gcol_elems, most);
-        if (st != CTFP_OK) return st;
+        // allocated once, for a call over every view; where memory is short, fewer
+        // sets (a larger rounding error) before an error
+        for (int k = accum_set_most(p->gp, p->gp.P, p->M); !p->d_gcol; k = (k + 1) / 2) {
+            const cudaError_t e = cudaMalloc(&p->d_gcol, sizeof(float) * prm.set_floats * k);
+            if (e == cudaSuccess) {
+                p->gcol_sets = k;
+                break;
+            }
+            if (e != cudaErrorMemoryAllocation || k == 1) return cuda_fail(e, "adjoint accumulators");
+            p->d_gcol = nullptr;
+            cudaGetLastError();  // not this call's error
+        }
+        prm.sets = accum_set_count(p->gp, prm.n_views, p->M, p->gcol_sets);
         prm.gcol = p->d_gcol;
         CTFP_CUDA(cudaMemsetAsync(prm.gcol, 0, sizeof(float) * prm.set_floats * prm.sets, s));
     }

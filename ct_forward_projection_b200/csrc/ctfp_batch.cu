@@ -474,6 +474,7 @@ struct ctfp_batch {
     unsigned long long* d_counter = nullptr;    // one per group
     float* d_gcol = nullptr;           // all items' accumulators, contiguous
     size_t gcol_floats = 0;
+    int most_sets = 0;                 // at most so many sets per item
     std::vector<size_t> gcol_off;      // [slot]
     cudaStream_t capture = nullptr;    // private stream the graphs are recorded on
     // one graph per kind, valid for the tables, volume pointers and loss
@@ -662,7 +663,8 @@ ctfp_status fill_items(ctfp_batch* b, int kind)
         it.tiles_v = (it.g.V + b->tile_v[kind] - 1) / b->tile_v[kind];
         it.vgroups = (it.g.P + b->vpu[kind] - 1) / b->vpu[kind];
         it.set_floats = accum_floats(it.g.nx, it.g.ny, it.g.nz, it.M);
-        it.set_groups = (it.vgroups + accum_sets(it.g, it.g.P, it.M) - 1) / accum_sets(it.g, it.g.P, it.M);
+        const int sets = accum_sets(it.g, it.g.P, it.M, b->most_sets);
+        it.set_groups = (it.vgroups + sets - 1) / sets;
         it.sets = (it.vgroups + it.set_groups - 1) / it.set_groups;
         it.unit0 = unit0;
         it.units = units;
@@ -720,7 +722,6 @@ ctfp_status ctfp_batch_create(int32_t n_items, ctfp_plan* const* plans, ctfp_bat
     b->tile0.resize((size_t)n_items);
     b->gcol_off.assign((size_t)n_items, 0);
     long long unit = 0, tiles = 0;
-    size_t gcol = 0;
     for (int s = 0; s < n_items; s++) {
         ctfp_plan* p = plans[b->order[(size_t)s]];
         const GeomParams& g = plan_geom(p);
@@ -735,17 +736,32 @@ ctfp_status ctfp_batch_create(int32_t n_items, ctfp_plan* const* plans, ctfp_bat
         b->groups.back().count++;
         b->tile0[(size_t)s] = tiles;
         tiles += column_tiles(g.nx, g.ny, g.nz);
-        b->gcol_off[(size_t)s] = gcol;
-        if (column_fits(g.nx, g.ny, g.nz)) gcol += (accum_floats(g.nx, g.ny, g.nz, it.M) * accum_sets(g, g.P, it.M) + 63) / 64 * 64;  // each item's on a 256-byte boundary
     }
     layout_units(b, 0);
     b->total_tiles = tiles;
-    b->gcol_floats = gcol;
     cudaError_t e = cudaMalloc(&b->d_items[0], sizeof(ItemDesc) * (size_t)n_items);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_items[1], sizeof(ItemDesc) * (size_t)n_items);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_tile0, sizeof(long long) * (size_t)n_items);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, sizeof(unsigned long long) * b->groups.size());
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_gcol, sizeof(float) * std::max<size_t>(gcol, 1));
+    // the accumulators; where memory is short, fewer sets of them for every item
+    for (int most = 8; e == cudaSuccess && !b->d_gcol; most /= 2) {
+        size_t gcol = 0;
+        for (int s = 0; s < n_items; s++) {
+            const GeomParams& g = plan_geom(plans[b->order[(size_t)s]]);
+            const int M = b->items[(size_t)s].M;
+            b->gcol_off[(size_t)s] = gcol;
+            if (column_fits(g.nx, g.ny, g.nz))  // each item's on a 256-byte boundary
+                gcol += (accum_floats(g.nx, g.ny, g.nz, M) * accum_sets(g, g.P, M, most) + 63) / 64 * 64;
+        }
+        b->gcol_floats = gcol;
+        b->most_sets = most;
+        e = cudaMalloc(&b->d_gcol, sizeof(float) * std::max<size_t>(gcol, 1));
+        if (e == cudaErrorMemoryAllocation && most > 1) {
+            b->d_gcol = nullptr;
+            cudaGetLastError();  // not this call's error
+            e = cudaSuccess;
+        }
+    }
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_tile0, b->tile0.data(), sizeof(long long) * (size_t)n_items, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);

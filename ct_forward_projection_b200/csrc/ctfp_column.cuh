@@ -4,6 +4,7 @@
 // persistent kernels.
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 
 #include "ctfp_axis.cuh"
@@ -289,20 +290,28 @@ __device__ __forceinline__ void march_axis(const GeomParams& g, const cudaTextur
 __host__ __device__ constexpr int accum_width(int M) { return M <= 2 ? 2 * M : 4; }
 
 // Sets of accumulators an adjoint over n views sums into (contiguous ranges of
-// the views, folded together): an FP32 sum of many small terms loses about
-// sqrt(terms) ulp of itself, and K sets of a K-th of the terms lose a K-th of
-// that.  At most as many as keep the gradients' error against FP64 at that of
-// separate accumulators per face corner and march axis (8 per voxel); fewer
-// where a voxel collects few rays (n views of one ray per voxel face each).
-// 2-norm relative error, one set / these sets / those 8: 97 x 113 x 75 voxels, 2
-// materials, 41 views 1.5e-7 / 6.4e-8 / 5.8e-8; 256^3, 3 materials, 90 views
-// 2.5e-7 / 1.1e-7 / 1.0e-7; 360 views, 2 materials (4 sets) 1.3e-7 against 1.2e-7.
-inline int accum_sets(const GeomParams& g, int n, int M)
+// the views, folded together in FP64): an FP32 sum of many small terms loses
+// about sqrt(terms) ulp of itself, and K sets of a K-th of the terms lose a K-th
+// of that.  As many as leave the gradients' error against FP64 no larger than
+// that of 8 separate accumulators per voxel (one per face corner and march
+// axis): 5 of pair cells, 8 of single voxels; and one per ray that meets a voxel
+// (n views of one ray per voxel face each).  2-norm relative error, 1 / 2 sums per
+// voxel in 4 or 6 sets / these / those 8: 97 x 113 x 75, 2 materials, 41 views
+// 1.5e-7 / 6.2e-8 / 4.9e-8 / 5.7e-8, 360 views - / 1.26e-7 / 1.01e-7 / 1.22e-7;
+// 256^3, 3 materials, 90 views 2.5e-7 / 1.06e-7 / 9.6e-8 / 1.00e-7; 64^3, 4 materials,
+// rays 0.37 voxels apart - / 1.66e-7 / 1.25e-7 / 1.26e-7.  Times are the same.
+inline int accum_most(const GeomParams& g, int n, int M)
 {
     const float pitch = g.dSize * g.sod / g.sdd;
     const float rays = (float)n * g.pSizeZ * fminf(g.pSizeX, g.pSizeY) / (pitch * pitch);
-    const int most = M <= 2 ? 4 : 6, k = rays < 6.f * most ? (int)ceilf(rays / 6.f) : most;
-    return k < 1 ? 1 : (k < n ? k : n);
+    const int most = M <= 2 ? 5 : 8;
+    return std::max(1, std::min(rays < (float)most ? (int)ceilf(rays) : most, n));
+}
+// The sets that n views are summed into, of at most `most` allocated ones.
+inline int accum_sets(const GeomParams& g, int n, int M, int most)
+{
+    const int k = std::min(accum_most(g, n, M), most), views = (n + k - 1) / k;  // views of a set
+    return (n + views - 1) / views;
 }
 
 __device__ __forceinline__ void red_v2(float* q, float a, float b)
@@ -550,25 +559,26 @@ __device__ __forceinline__ void fold_tile(const float* __restrict__ acc, int set
         if (x < nx && z < nz) {
             const float* q =
                 acc + ((size_t)x * cd.sx + (size_t)y * cd.sy + (size_t)z + cd.origin) * accum_width(M);
-            // pair cells: voxel z is the first half of cell z and the second of cell z - 1
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            // pair cells: voxel z is the first half of cell z and the second of cell z - 1;
+            // in FP64, so that only the sums themselves have been rounded
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
             for (int j = 0; j < sets; j++, q += stride) {
                 if (M == 1) {
-                    v[0] += q[0] + q[-1];
+                    v[0] += (double)q[0] + (double)q[-1];
                 } else if (M == 2) {
                     const float2 e = *(const float2*)q, f = *(const float2*)(q - 2);
-                    v[0] += e.x + f.x;
-                    v[1] += e.y + f.y;
+                    v[0] += (double)e.x + (double)f.x;
+                    v[1] += (double)e.y + (double)f.y;
                 } else {
                     const float4 e = *(const float4*)q;
-                    v[0] += e.x;
-                    v[1] += e.y;
-                    v[2] += e.z;
-                    v[3] += e.w;
+                    v[0] += (double)e.x;
+                    v[1] += (double)e.y;
+                    v[2] += (double)e.z;
+                    v[3] += (double)e.w;
                 }
             }
 #pragma unroll
-            for (int m = 0; m < M; m++) t[m][tx][k] = v[m];
+            for (int m = 0; m < M; m++) t[m][tx][k] = (float)v[m];
         }
     }
     __syncthreads();

@@ -1340,7 +1340,9 @@ cudaError_t launch_spectral_from_L(const MarchParams& prm, int M, cudaStream_t s
 
 bool accum_fits(int nx, int ny, int nz) { return column_fits(nx, ny, nz); }
 
-int accum_set_count(const GeomParams& g, int n_views, int M) { return accum_sets(g, n_views, M); }
+int accum_set_most(const GeomParams& g, int n_views, int M) { return accum_most(g, n_views, M); }
+
+int accum_set_count(const GeomParams& g, int n_views, int M, int most) { return accum_sets(g, n_views, M, most); }
 
 size_t accum_floats(int nx, int ny, int nz, int M) { return column_dims(nx, ny, nz).elems * accum_width(M); }
 
@@ -1372,7 +1374,8 @@ cudaError_t launch_backward(const MarchParams& prm_in, int M, int interp, bool f
     const unsigned tiles_u = (unsigned)((prm_in.g.U + bs.tile_u - 1) / bs.tile_u);
     // view groups run along grid.y, at most 65535 per launch: all sets in one
     // launch, or past that one part of a set's views after the other
-    const int vpc = ls.views_per_cta, sets = prm_in.gcol ? prm_in.sets : 1;
+    const int sets = prm_in.gcol ? prm_in.sets : 1;
+    const int vpc = std::max(1, std::min(ls.views_per_cta, prm_in.n_views / sets));  // few views: still every set
     const int groups = (prm_in.n_views + vpc - 1) / vpc;
     b.set_groups = (groups + sets - 1) / sets;
     const bool whole = b.set_groups <= 65535;

@@ -64,7 +64,8 @@ cudaError_t launch_forward(const MarchParams& prm, int M, int interp, int sample
 cudaError_t launch_spectral_from_L(const MarchParams& prm, int M, cudaStream_t st);
 // Floats of one set of the adjoint's accumulators (accum_width).
 size_t accum_floats(int nx, int ny, int nz, int M);
-int accum_set_count(const GeomParams& g, int n_views, int M);  // accum_sets
+int accum_set_most(const GeomParams& g, int n_views, int M);  // accum_most
+int accum_set_count(const GeomParams& g, int n_views, int M, int most);  // accum_sets
 bool accum_fits(int nx, int ny, int nz);  // false: launch_backward adds into prm.gvol (prm.gcol null)
 // Adjoint scatter into the accumulators prm.gcol (zeroed by the caller),
 // followed by launch_fold into prm.gvol.
