@@ -370,7 +370,8 @@ __global__ void __launch_bounds__(256) k_spectral_from_L(const MarchParams prm)
     const int64_t n = per_view * prm.g.P, stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += stride) {
         const int64_t p = t / per_view;
-        const int r = (int)(t - p * per_view), block = r >> 5, lane = r & 31;
+        const int64_t r = t - p * per_view;  // over 2^31 for a detector of 65535 x 32769 and more
+        const int block = (int)(r >> 5), lane = (int)(r & 31);
         const int u = (block % bu) * 4 + (lane & 3), v = (block / bu) * 8 + (lane >> 2);
         if (u >= prm.g.U || v >= prm.g.V) continue;
         const int64_t ray = p * npix + (int64_t)v * prm.g.U + u;
