@@ -521,12 +521,12 @@ __device__ __forceinline__ void scatter_columns(const GeomParams& gp, float* acc
 }
 
 // The same for a volume that column_fits refuses: every voxel of every sample
-// by an atomic addition into the gradients.
+// by an atomic addition into the gradients.  A batch's tuning runs have none.
 template <int M, int MODE>
 __device__ __noinline__ void scatter_direct(const GeomParams& gp, float* const* gvol, bool on, int p, int v, int u,
                                             const float* g)
 {
-    if (!on) return;
+    if (!on || !gvol[0]) return;
     const RaySeg s = ray_segment(gp, p, v, u);
     const RayRef32 r = ray_ref32(gp, p, v, u);
     for (int i = s.i0; i < s.i1; i++) {
