@@ -32,7 +32,7 @@ struct ctfp_plan {
     int E = 0;
     bool spectral_ready = false;
     float* d_mu = nullptr;  // [E][M]
-    float* d_W = nullptr;   // energy weights (weight_index)
+    float* d_W = nullptr;   // energy weights (pixel_weights)
     float* d_I0 = nullptr;  // [V][U]
     // texture mode
     cudaArray_t arr[kMaxM] = {};

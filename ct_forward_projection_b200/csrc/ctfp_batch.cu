@@ -79,7 +79,7 @@ struct ItemDesc {
     cudaTextureObject_t tex[kMaxM];    // 3D textures (TEXTURE: the reference's own sampler)
     const float* cvol; // the axis sampler's column copy (four materials)
     const float* mu;   // [E][M]
-    const float* W;    // energy weights (weight_index)
+    const float* W;    // energy weights (pixel_weights)
     int M, E, interp;
     int tiles_u, tiles_v;
     int vgroups;       // groups of views per unit: ceil(P / views per unit)

@@ -496,22 +496,34 @@ __device__ __forceinline__ void kahan_join(float& s, float& c, float s2, float c
 // With a plain [E][V][U] table a warp of 4 columns loaded 16 bytes of each of 8
 // rows per energy.  Measured, plain table -> blocks: 128^3, 1 material, 61
 // energies, forward 2.107 -> 1.996 ms; 256^3, 101 energies, 2 materials, forward
-// 48.27 -> 47.9 ms, 3 materials, training step 29.7 -> 28.7 ms.  Element (e, v, u) is float
-// ((block * E4 + e / 4) * 32 + lane) * 4 + e % 4, E4 = ceil(E / 4).
+// 48.27 -> 47.9 ms, 3 materials, training step 29.7 -> 28.7 ms.  The last E % 4
+// energies are not padded to a group (one energy would take four times its
+// bytes): element (e, v, u) is float block * 32 E + 128 (e / 4) + 4 lane + e % 4,
+// and from e = 4 (E / 4) on block * 32 E + 32 e + lane.
 __host__ __device__ __forceinline__ int energy_groups(int E) { return (E + 3) >> 2; }
 __host__ __device__ __forceinline__ size_t weight_floats(int U, int V, int E)
 {
-    return (size_t)((U + 3) >> 2) * (size_t)((V + 7) >> 3) * (size_t)energy_groups(E) * 128;
+    return (size_t)((U + 3) >> 2) * (size_t)((V + 7) >> 3) * (size_t)E * 32;
 }
-__host__ __device__ __forceinline__ size_t weight_index(int U, int E, int u, int v)
+// One pixel's weights: group g of 4 energies is full[g * 32], energy e past the
+// last full group rest[e * 32].
+template <class F4, class F>
+struct PixelWeightsT {
+    F4* full;
+    F* rest;
+};
+using PixelWeights = PixelWeightsT<const float4, const float>;
+template <class F4, class F>
+__device__ __forceinline__ PixelWeightsT<F4, F> pixel_weights_at(F* W, int U, int E, int u, int v)
 {
     const size_t block = (size_t)(v >> 3) * (size_t)((U + 3) >> 2) + (size_t)(u >> 2);
-    return (block * (size_t)energy_groups(E) * 32 + (size_t)((v & 7) * 4 + (u & 3))) * 4;
+    F* at = W + block * (size_t)E * 32;
+    const int lane = (v & 7) * 4 + (u & 3);
+    return {(F4*)at + lane, at + lane};
 }
-// One pixel's weights: group e4 is element e4 * 32.
-__device__ __forceinline__ const float4* pixel_weights(const float* W, int U, int E, int u, int v)
+__device__ __forceinline__ PixelWeights pixel_weights(const float* W, int U, int E, int u, int v)
 {
-    return (const float4*)(W + weight_index(U, E, u, v));
+    return pixel_weights_at<const float4>(W, U, E, u, v);
 }
 // The attenuation table in shared memory: [M][E4 * 4], a group's 4 energies of a
 // material in one 16-byte load; the pad holds 0.
@@ -526,14 +538,14 @@ __device__ __forceinline__ void stage_mu(float* s_mu, const float* __restrict__ 
 // for the last E % 4), att = sum_m mu[e][m] L[m].  Two groups per step: two
 // weight loads in flight.
 template <int M, class Term>
-__device__ __forceinline__ void for_energies(const float* s_mu, int E, const float4* __restrict__ Wp, const float* L,
+__device__ __forceinline__ void for_energies(const float* s_mu, int E, const PixelWeights& W, const float* L,
                                              Term term)
 {
     const int E4 = energy_groups(E), full = E >> 2;
     const float4* mu4 = (const float4*)s_mu;
 #pragma unroll 2
     for (int g = 0; g < full; g++) {
-        const float4 w = __ldg(Wp + g * 32);
+        const float4 w = __ldg(W.full + g * 32);
         float att[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int m = 0; m < M; m++) {
@@ -552,7 +564,7 @@ __device__ __forceinline__ void for_energies(const float* s_mu, int E, const flo
         float att = 0.f;
 #pragma unroll
         for (int m = 0; m < M; m++) att = fmaf(s_mu[m * E4 * 4 + e], L[m], att);
-        term(0, e, att, __ldg((const float*)(Wp + full * 32) + (e & 3)));
+        term(0, e, att, __ldg(W.rest + e * 32));
     }
 }
 
@@ -562,11 +574,11 @@ __device__ __forceinline__ void for_energies(const float* s_mu, int E, const flo
 // relative rounding error stays below (E / 4 + 2) ulp with one fused
 // multiply-add per term and output.
 template <int M>
-__device__ __forceinline__ void spectral(const float* s_mu, int E, const float4* __restrict__ Wp, const float* L, float& I,
+__device__ __forceinline__ void spectral(const float* s_mu, int E, const PixelWeights& W, const float* L, float& I,
                                          float& IAbs)
 {
     float sI[4] = {0.f, 0.f, 0.f, 0.f}, sA[4] = {0.f, 0.f, 0.f, 0.f};
-    for_energies<M>(s_mu, E, Wp, L, [&](int k, int, float att, float w) {
+    for_energies<M>(s_mu, E, W, L, [&](int k, int, float att, float w) {
         float ex, om;
         transmit(att, ex, om);
         sI[k] = fmaf(w, ex, sI[k]);
@@ -580,14 +592,14 @@ __device__ __forceinline__ void spectral(const float* s_mu, int E, const float4*
 // (the same terms in the same order, so the batch's I equals the plain
 // forward's), and S_m = sum_e mu_em W_e exp(-a_e), the derivative -dI/dL_m.
 template <int M>
-__device__ __forceinline__ void spectral_adjoint(const float* s_mu, int E, const float4* __restrict__ Wp, const float* L,
+__device__ __forceinline__ void spectral_adjoint(const float* s_mu, int E, const PixelWeights& W, const float* L,
                                                  float& I, float* S)
 {
     float sI[4] = {0.f, 0.f, 0.f, 0.f};
     const int Ep = energy_groups(E) * 4;
 #pragma unroll
     for (int m = 0; m < M; m++) S[m] = 0.f;
-    for_energies<M>(s_mu, E, Wp, L, [&](int k, int e, float att, float w) {
+    for_energies<M>(s_mu, E, W, L, [&](int k, int e, float att, float w) {
         float ex, om;
         transmit(att, ex, om);
         sI[k] = fmaf(w, ex, sI[k]);

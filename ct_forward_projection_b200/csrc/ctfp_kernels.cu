@@ -235,23 +235,23 @@ __global__ void __launch_bounds__(128, uses_columns(M) ? 6 : 8) k_forward_axis_s
         const int first = shift == 1 ? 2 * part : part, own = shift == 1 ? 2 : 1;
         float sI = 0.f, sA = 0.f;
         if (on && first < 4) {
-            const float* Wp = (const float*)pixel_weights(prm.W, prm.g.U, prm.E, u, v);
+            const PixelWeights W = pixel_weights(prm.W, prm.g.U, prm.E, u, v);
             const int full = prm.E >> 2, Ep = energy_groups(prm.E) * 4;
             for (int a = 0; a < own; a++) {
                 float tI = 0.f, tA = 0.f;
-                const auto term = [&](int e) {
+                const auto term = [&](int e, const float* at) {
                     float att = 0.f, ex, om;
 #pragma unroll
                     for (int m = 0; m < M; m++) att = fmaf(s_mu[m * Ep + e], L[m], att);
-                    const float w = __ldg(Wp + (e >> 2) * 128 + (e & 3));
+                    const float w = __ldg(at);
                     transmit(att, ex, om);
                     tI = fmaf(w, ex, tI);
                     tA = fmaf(w, om, tA);
                 };
 #pragma unroll 4
-                for (int g = 0; g < full; g++) term(4 * g + first + a);
+                for (int g = 0; g < full; g++) term(4 * g + first + a, (const float*)(W.full + g * 32) + first + a);
                 if (first + a == 0)
-                    for (int e = 4 * full; e < prm.E; e++) term(e);
+                    for (int e = 4 * full; e < prm.E; e++) term(e, W.rest + e * 32);
                 sI += tI;
                 sA += tA;
             }
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(256) k_fold(const MarchParams prm)
 }
 
 // W[e][k] = ((I0Val * S_e) * G_e) * D_e in the reference's multiplication order
-// (CBCTPolyProjGPU.cu:1994), laid out as weight_index; I0[k] = the sum over e
+// (CBCTPolyProjGPU.cu:1994), laid out as pixel_weights reads it; I0[k] = the sum over e
 // (CBCTPolyForwardProjGrid.cpp:330-339).
 __global__ void k_weights(const float* __restrict__ S, const float* __restrict__ G, int grid_layout,
                           const float* __restrict__ D, float I0Val, int E, int U, int V, float* W, float* I0)
@@ -484,24 +484,28 @@ __global__ void k_weights(const float* __restrict__ S, const float* __restrict__
         // accumulator 0, combined pairwise), so that a ray with no attenuation
         // gives exactly I0
         float s[4] = {0.f, 0.f, 0.f, 0.f};
-        float4* Wp = (float4*)(W + weight_index(U, E, u, v));
-        const int E4 = energy_groups(E);
-        for (int g = 0; g < E4; g++) {
+        const auto Wp = pixel_weights_at<float4>(W, U, E, u, v);
+        const auto weight = [&](int e) {
+            float w = I0Val * S[e];
+            if (grid_layout == 1) w = w * G[(int64_t)e * U + u];
+            if (grid_layout == 2) w = w * G[(int64_t)e * npix + k];
+            if (D) w = w * D[(int64_t)e * npix + k];
+            return w;
+        };
+        const int full = E >> 2;
+        for (int g = 0; g < full; g++) {
             float w[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const int e = 4 * g + j;
-                w[j] = 0.f;
-                if (e < E) {
-                    w[j] = I0Val * S[e];
-                    if (grid_layout == 1) w[j] = w[j] * G[(int64_t)e * U + u];
-                    if (grid_layout == 2) w[j] = w[j] * G[(int64_t)e * npix + k];
-                    if (D) w[j] = w[j] * D[(int64_t)e * npix + k];
-                    if (4 * g + 4 <= E) s[j] += w[j];
-                    else s[0] += w[j];
-                }
+                w[j] = weight(4 * g + j);
+                s[j] += w[j];
             }
-            Wp[g * 32] = make_float4(w[0], w[1], w[2], w[3]);
+            Wp.full[g * 32] = make_float4(w[0], w[1], w[2], w[3]);
+        }
+        for (int e = 4 * full; e < E; e++) {
+            const float w = weight(e);
+            s[0] += w;
+            Wp.rest[e * 32] = w;
         }
         I0[k] = (s[0] + s[1]) + (s[2] + s[3]);
     }

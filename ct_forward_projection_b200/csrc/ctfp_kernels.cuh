@@ -18,7 +18,7 @@ struct MarchParams {
     const float* Lin;                 // [P][V][U][M] path integrals (in, epilogue/adjoint)
     float* I;                         // [P][V][U] (may be null)
     float* IAbs;                      // [P][V][U] (may be null)
-    const float* W;                   // energy weights I0Val*S*G*D of every pixel (weight_index)
+    const float* W;                   // energy weights I0Val*S*G*D of every pixel (pixel_weights)
     const float* mu;                  // [E][M] attenuation per density, 1/mm per g/cm^3
     const float* gI;                  // [P][V][U] dLoss/dI (adjoint)
     const float* gIAbs;               // [P][V][U] dLoss/dIAbsorb (adjoint, may be null)
