@@ -423,7 +423,7 @@ ctfp_status scatter_and_fold(ctfp_plan* p, MarchParams prm, bool from_gL, cudaSt
         prm.set_floats = accum_floats(p->gp.nx, p->gp.ny, p->gp.nz, p->M);
         // allocated once, for a call over every view; where memory is short, fewer
         // sets (a larger rounding error) before an error
-        for (int k = accum_set_most(p->gp, p->gp.P, p->M); !p->d_gcol; k = (k + 1) / 2) {
+        for (int k = accum_set_count(p->gp, p->gp.P, p->M); !p->d_gcol; k = (k + 1) / 2) {
             const cudaError_t e = cudaMalloc(&p->d_gcol, sizeof(float) * prm.set_floats * k);
             if (e == cudaSuccess) {
                 p->gcol_sets = k;
@@ -433,7 +433,7 @@ ctfp_status scatter_and_fold(ctfp_plan* p, MarchParams prm, bool from_gL, cudaSt
             p->d_gcol = nullptr;
             cudaGetLastError();  // not this call's error
         }
-        prm.sets = accum_set_count(p->gp, prm.n_views, p->M, p->gcol_sets);
+        set_accum_sets(prm, p->M, p->gcol_sets);
         prm.gcol = p->d_gcol;
         CTFP_CUDA(cudaMemsetAsync(prm.gcol, 0, sizeof(float) * prm.set_floats * prm.sets, s));
     }

@@ -92,7 +92,7 @@ struct ItemDesc {
     const float* I_target;
     float* gvol[kMaxM];
     float* gcol;       // accumulators of every material (ctfp_column.cuh); null: gvol takes the sums directly
-    int sets, set_groups;  // sets of accumulators, and the view groups that sum into one (accum_sets)
+    int sets, set_parts;  // sets of accumulators and the parts of the view groups (accum_sets)
     size_t set_floats;
     float* loss;       // device scalar accumulated with atomicAdd
 };
@@ -255,7 +255,10 @@ __device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M
     // emulation reproduces exactly (as ctfp_backward does for such a plan)
     constexpr int SM = MODE == INTERP_TRILINEAR ? INTERP_TRILINEAR : INTERP_TEXEMU;
     if (!AXIS && !it.gcol) scatter_direct<M, SM>(it.g, it.gvol, any, p, v, u, g);
-    else scatter_columns<M, SM, (M > 2 && MODE == INTERP_TRILINEAR)>(it.g, it.gcol + (size_t)set * it.set_floats, any, p, v, u, g);
+    else {
+        const int cols = it.sets / it.set_parts, at = set * cols + (u & (cols - 1));
+        scatter_columns<M, SM, (M > 2 && MODE == INTERP_TRILINEAR)>(it.g, it.gcol + (size_t)at * it.set_floats, any, p, v, u, g);
+    }
     return res * res;
 }
 
@@ -327,7 +330,7 @@ __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJO
                     const int rem = (int)(local % band_units);
                     s_tv = (int)(local / band_units);
                     s_p = rem / it.tiles_u;
-                    s_set = s_p / it.set_groups;
+                    s_set = (int)((long long)s_p * it.set_parts / it.vgroups);
                     s_tu = rem % it.tiles_u;
                 } else {
                     const int tiles = it.tiles_u * it.tiles_v;
@@ -663,9 +666,9 @@ ctfp_status fill_items(ctfp_batch* b, int kind)
         it.tiles_v = (it.g.V + b->tile_v[kind] - 1) / b->tile_v[kind];
         it.vgroups = (it.g.P + b->vpu[kind] - 1) / b->vpu[kind];
         it.set_floats = accum_floats(it.g.nx, it.g.ny, it.g.nz, it.M);
-        const int sets = accum_sets(it.g, it.g.P, it.M, b->most_sets);
-        it.set_groups = (it.vgroups + sets - 1) / sets;
-        it.sets = (it.vgroups + it.set_groups - 1) / it.set_groups;
+        const AccumSets sets = accum_sets(it.g, it.g.P, it.M, b->most_sets);
+        it.set_parts = std::min(it.vgroups, sets.views);
+        it.sets = it.set_parts * sets.columns;
         it.unit0 = unit0;
         it.units = units;
     }
@@ -744,14 +747,14 @@ ctfp_status ctfp_batch_create(int32_t n_items, ctfp_plan* const* plans, ctfp_bat
     if (e == cudaSuccess) e = cudaMalloc(&b->d_tile0, sizeof(long long) * (size_t)n_items);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, sizeof(unsigned long long) * b->groups.size());
     // the accumulators; where memory is short, fewer sets of them for every item
-    for (int most = 8; e == cudaSuccess && !b->d_gcol; most /= 2) {
+    for (int most = kMostSets; e == cudaSuccess && !b->d_gcol; most /= 2) {
         size_t gcol = 0;
         for (int s = 0; s < n_items; s++) {
             const GeomParams& g = plan_geom(plans[b->order[(size_t)s]]);
             const int M = b->items[(size_t)s].M;
             b->gcol_off[(size_t)s] = gcol;
             if (column_fits(g.nx, g.ny, g.nz))  // each item's on a 256-byte boundary
-                gcol += (accum_floats(g.nx, g.ny, g.nz, M) * accum_sets(g, g.P, M, most) + 63) / 64 * 64;
+                gcol += (accum_floats(g.nx, g.ny, g.nz, M) * accum_sets(g, g.P, M, most).total() + 63) / 64 * 64;
         }
         b->gcol_floats = gcol;
         b->most_sets = most;

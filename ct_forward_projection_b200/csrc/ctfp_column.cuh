@@ -289,30 +289,47 @@ __device__ __forceinline__ void march_axis(const GeomParams& g, const cudaTextur
 // views, 1 material 3.2 -> 2.4 ms; 512^3, 48 views, 4 materials 558 -> 260 ms.
 __host__ __device__ constexpr int accum_width(int M) { return M <= 2 ? 2 * M : 4; }
 
-// Sets of accumulators an adjoint over n views sums into (contiguous ranges of
-// the views, folded together in FP64): an FP32 sum of many small terms loses
-// about sqrt(terms) ulp of itself, and K sets of a K-th of the terms lose a K-th
-// of that.  As many as leave the gradients' error against FP64 no larger than
-// that of 8 separate accumulators per voxel (one per face corner and march
-// axis): 5 of pair cells, 8 of single voxels; and one per ray that meets a voxel
-// (n views of one ray per voxel face each).  2-norm relative error, 1 / 2 sums per
-// voxel in 4 or 6 sets / these / those 8: 97 x 113 x 75, 2 materials, 41 views
-// 1.5e-7 / 6.2e-8 / 4.9e-8 / 5.7e-8, 360 views - / 1.26e-7 / 1.01e-7 / 1.22e-7;
-// 256^3, 3 materials, 90 views 2.5e-7 / 1.06e-7 / 9.6e-8 / 1.00e-7; 64^3, 4 materials,
-// rays 0.37 voxels apart - / 1.66e-7 / 1.25e-7 / 1.26e-7.  Times are the same.
-inline int accum_most(const GeomParams& g, int n, int M)
+// Sets of accumulators an adjoint over n views sums into, folded together in
+// FP64: views equal parts of the views, by columns of the detector within each.
+// An FP32 sum of many small terms loses about sqrt(terms) ulp of itself, and K
+// sets of a K-th of the terms lose a K-th (positive terms) to a sqrt(K)-th
+// (signed ones) of that.  As many as leave the gradients' error against FP64 no
+// larger than that of 8 separate accumulators per voxel, one per face corner and
+// march axis, which took each a share of every view's rays: the more, the more
+// rays of one view meet a voxel's face, the fewer, the fewer views there are; and
+// where a view's rays alone outnumber what the views can be split into, its
+// columns take turns.  2-norm relative error of 4 / 5 / 6 / 7 / 8 sets of single voxels
+// against those 8: 256^3, 0.6 rays a face, 90 views 11.4 10.6 10.2 10.0 9.8 /
+// 10.4e-8; 128^3, 4.1, 53 views 15.9 14.3 13.3 12.5 12.1 / 12.5e-8; 66^3, 19, 182
+// views 56 45 38 33 29.9 / 28.8e-8; 65^3, 74, 7 views 27 24 22 17.7 - / 15.7e-8.
+// Pair cells hold two sums a voxel: 48^3, 8.2 rays, 60 views, 4 / 5 / 6 sets 36 32
+// 29 / 32e-8, 1 ray, 13.9 12.8 11.9 / 13.4e-8; 20 views 9.4 8.8 8.4 / 9.6e-8, 7 views 3
+// sets 7.9 / 8.1e-8.
+struct AccumSets {
+    int views, columns;
+    int total() const { return views * columns; }
+};
+inline AccumSets accum_sets(const GeomParams& g, int n, int M, int most)
 {
-    const float pitch = g.dSize * g.sod / g.sdd;
-    const float rays = (float)n * g.pSizeZ * fminf(g.pSizeX, g.pSizeY) / (pitch * pitch);
-    const int most = M <= 2 ? 5 : 8;
-    return std::max(1, std::min(rays < (float)most ? (int)ceilf(rays) : most, n));
+    const float pitch = g.dSize * g.sod / g.sdd, across = fminf(g.pSizeX, g.pSizeY);
+    const float face = g.pSizeZ * across / (pitch * pitch), rays = fminf((float)n * face, 1e6f);
+    const int full = M <= 2 ? (face > 8.f ? 6 : 5) : (face > 8.f ? 10 : face > 1.7f ? 8 : 6);
+    int k = full;
+    if (face <= 1.7f) {
+        int lg = 1;  // 1 + floor(log2 n)
+        for (int j = n; j > 1; j >>= 1) lg++;
+        if (face < 0.3f && lg > 3) lg--;
+        k = std::max(std::min(k, lg), std::min((int)ceilf(rays / 6.f), M <= 2 ? 4 : 6));
+    }
+    AccumSets s;
+    s.views = std::max(1, std::min(std::min(k, (int)ceilf(rays) + 1), std::min(n, most)));
+    s.columns = 1;
+    const int want = M <= 2 ? 2 : full;
+    if (face > 1.7f && pitch < 0.75f * across)
+        while (s.columns < 4 && 6 * s.total() < 5 * want && 2 * s.total() <= most) s.columns *= 2;
+    return s;
 }
-// The sets that n views are summed into, of at most `most` allocated ones.
-inline int accum_sets(const GeomParams& g, int n, int M, int most)
-{
-    const int k = std::min(accum_most(g, n, M), most), views = (n + k - 1) / k;  // views of a set
-    return (n + views - 1) / views;
-}
+constexpr int kMostSets = 18;  // more than any plan's
 
 __device__ __forceinline__ void red_v2(float* q, float a, float b)
 {

@@ -392,8 +392,8 @@ __global__ void __launch_bounds__(256, 6) k_spectral_from_L(const MarchParams pr
 // reductions.  FROM_GL: the input is dLoss/dL directly (transpose of the line
 // integrals).
 //
-// Grid: x = pixel tiles along u, y = the view groups of a set of accumulators,
-// z = pixel tiles along v of every set, so that the CTAs resident at any time
+// Grid: x = pixel tiles along u, y = the view groups of one part of the views,
+// z = pixel tiles along v of every part, so that the CTAs resident at any time
 // cover one band of detector rows for many views.  The rays of a row band cross a thin z-slab of the volume (the cone
 // angle is small), so the accumulator cells they reduce into stay in L2; with
 // views outermost every view would sweep the whole accumulator through DRAM.
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(256, 6) k_spectral_from_L(const MarchParams pr
 enum { kEach, kMerge, kDirect };
 template <int M, int MODE, bool FROM_GL, int KIND>
 __global__ void __launch_bounds__(256, 4)
-    k_backward(const MarchParams prm, int tile_u, int warp_rows, int tiles_v, int set_groups)
+    k_backward(const MarchParams prm, int tile_u, int warp_rows, int tiles_v, int group0)
 {
     extern __shared__ __align__(16) float s_mu[];
     if (!FROM_GL) load_mu(s_mu, prm.mu, prm.E, M);
@@ -412,14 +412,18 @@ __global__ void __launch_bounds__(256, 4)
     const int tile_v = (int)blockDim.x / tile_u;
     const int wcols = 32 / warp_rows, warps_u = tile_u / wcols;
     const int u = blockIdx.x * tile_u + (w % warps_u) * wcols + lane / warp_rows;
-    const int set = blockIdx.z / tiles_v, band = blockIdx.z % tiles_v;
+    const int part = blockIdx.z / tiles_v, band = blockIdx.z % tiles_v;
     const int v = band * tile_v + (w / warps_u) * warp_rows + lane % warp_rows;
     const bool ray_on = u < prm.g.U && v < prm.g.V;
     const int64_t npix = (int64_t)prm.g.U * prm.g.V;
     const int64_t pix = (int64_t)v * prm.g.U + u;
-    const int pend = prm.view0 + prm.n_views;
+    // the part's views, each part's as many as another's or one more
+    const int parts = prm.sets / prm.set_columns;
+    const int first = prm.view0 + (int)((int64_t)prm.n_views * part / parts);
+    const int pend = prm.view0 + (int)((int64_t)prm.n_views * (part + 1) / parts);
+    const int set = part * prm.set_columns + (u & (prm.set_columns - 1));
     for (int k = 0; k < prm.views_per_cta; k++) {
-        const int p = prm.view0 + (set * set_groups + blockIdx.y) * prm.views_per_cta + k;
+        const int p = first + (group0 + blockIdx.y) * prm.views_per_cta + k;
         if (p >= pend) break;
         const int64_t ray = (int64_t)(p - prm.out_view0) * npix + pix;
         float g[M];
@@ -1102,7 +1106,7 @@ bool merge_faces(const GeomParams& g, int interp)
 }
 
 struct BwdGrid {
-    int tile_u, rows, tiles_v, set_groups;
+    int tile_u, rows, tiles_v, group0;
     dim3 grid, block;
     size_t smem;
 };
@@ -1114,7 +1118,7 @@ cudaError_t bwd_launch(const MarchParams& prm, const BwdGrid& b, cudaStream_t st
     auto k = k_backward<M, MODE, FROM_GL, kEach>;
     if (!prm.gcol) k = k_backward<M, MODE, FROM_GL, kDirect>;
     else if (M > 2 && merge_faces(prm.g, MODE)) k = k_backward<M, MODE, FROM_GL, (M > 2 ? kMerge : kEach)>;
-    k<<<b.grid, b.block, smem, st>>>(prm, b.tile_u, b.rows, b.tiles_v, b.set_groups);
+    k<<<b.grid, b.block, smem, st>>>(prm, b.tile_u, b.rows, b.tiles_v, b.group0);
     return cudaGetLastError();
 }
 
@@ -1351,9 +1355,14 @@ cudaError_t launch_spectral_from_L(const MarchParams& prm, int M, cudaStream_t s
 
 bool accum_fits(int nx, int ny, int nz) { return column_fits(nx, ny, nz); }
 
-int accum_set_most(const GeomParams& g, int n_views, int M) { return accum_most(g, n_views, M); }
+int accum_set_count(const GeomParams& g, int n_views, int M) { return accum_sets(g, n_views, M, kMostSets).total(); }
 
-int accum_set_count(const GeomParams& g, int n_views, int M, int most) { return accum_sets(g, n_views, M, most); }
+void set_accum_sets(MarchParams& prm, int M, int most)
+{
+    const AccumSets s = accum_sets(prm.g, prm.n_views, M, most);
+    prm.sets = s.total();
+    prm.set_columns = s.columns;
+}
 
 size_t accum_floats(int nx, int ny, int nz, int M) { return column_dims(nx, ny, nz).elems * accum_width(M); }
 
@@ -1383,23 +1392,14 @@ cudaError_t launch_backward(const MarchParams& prm_in, int M, int interp, bool f
     b.block = dim3(threads);
     b.smem = sizeof(float) * (size_t)energy_groups(prm_in.E) * 4 * M;
     const unsigned tiles_u = (unsigned)((prm_in.g.U + bs.tile_u - 1) / bs.tile_u);
-    // view groups run along grid.y, at most 65535 per launch: all sets in one
-    // launch, or past that one part of a set's views after the other
-    const int sets = prm_in.gcol ? prm_in.sets : 1;
-    const int vpc = std::max(1, std::min(ls.views_per_cta, prm_in.n_views / sets));  // few views: still every set
-    const int groups = (prm_in.n_views + vpc - 1) / vpc;
-    b.set_groups = (groups + sets - 1) / sets;
-    const bool whole = b.set_groups <= 65535;
-    const int most = whole ? groups : 65535;
-    for (int g0 = 0; g0 < groups;) {
-        MarchParams prm = prm_in;
-        const int set = whole ? 0 : g0 / b.set_groups;
-        const int n = whole ? groups : std::min(std::min(most, groups - g0), (set + 1) * b.set_groups - g0);
-        prm.views_per_cta = vpc;
-        prm.view0 = prm_in.view0 + g0 * vpc;
-        prm.n_views = std::min(n * vpc, prm_in.n_views - g0 * vpc);
-        if (prm.gcol) prm.gcol += (size_t)set * prm.set_floats;
-        b.grid = whole ? dim3(tiles_u, b.set_groups, b.tiles_v * sets) : dim3(tiles_u, n, b.tiles_v);
+    // a part's view groups run along grid.y, at most 65535 per launch
+    MarchParams prm = prm_in;
+    if (!prm.gcol) prm.sets = prm.set_columns = 1;
+    const int parts = prm.sets / prm.set_columns, views = (prm.n_views + parts - 1) / parts;  // of the largest part
+    prm.views_per_cta = std::max(1, std::min(ls.views_per_cta, views));
+    const int groups = (views + prm.views_per_cta - 1) / prm.views_per_cta;
+    for (b.group0 = 0; b.group0 < groups; b.group0 += 65535) {
+        b.grid = dim3(tiles_u, std::min(65535, groups - b.group0), b.tiles_v * parts);
         if (b.grid.x == 0 || b.grid.y == 0 || b.grid.z == 0) return cudaSuccess;
         cudaError_t e = cudaErrorInvalidValue;
         switch (M) {
@@ -1409,7 +1409,6 @@ cudaError_t launch_backward(const MarchParams& prm_in, int M, int interp, bool f
             case 4: e = bwd_dispatch<4>(prm, interp, from_gL, b, st); break;
         }
         if (e != cudaSuccess) return e;
-        g0 += n;
     }
     return cudaSuccess;
 }

@@ -24,7 +24,8 @@ struct MarchParams {
     const float* gIAbs;               // [P][V][U] dLoss/dIAbsorb (adjoint, may be null)
     float* gvol[kMaxM];               // gradient volumes (adjoint)
     float* gcol;                      // gradient accumulators of every material (adjoint, ctfp_column.cuh)
-    int sets;                         // sets of them, set_floats apart, the views in as many contiguous parts
+    int sets;                         // sets of them, set_floats apart: as many parts of the views as
+    int set_columns;                  // set_columns (a power of two) goes into, times columns taking turns (accum_sets)
     size_t set_floats;
     int E;
     int view0;                        // first view of this launch
@@ -64,8 +65,8 @@ cudaError_t launch_forward(const MarchParams& prm, int M, int interp, int sample
 cudaError_t launch_spectral_from_L(const MarchParams& prm, int M, cudaStream_t st);
 // Floats of one set of the adjoint's accumulators (accum_width).
 size_t accum_floats(int nx, int ny, int nz, int M);
-int accum_set_most(const GeomParams& g, int n_views, int M);  // accum_most
-int accum_set_count(const GeomParams& g, int n_views, int M, int most);  // accum_sets
+int accum_set_count(const GeomParams& g, int n_views, int M);  // accum_sets, any number of sets
+void set_accum_sets(MarchParams& prm, int M, int most);        // prm.sets and prm.set_columns for prm.n_views, at most so many
 bool accum_fits(int nx, int ny, int nz);  // false: launch_backward adds into prm.gvol (prm.gcol null)
 // Adjoint scatter into the accumulators prm.gcol (zeroed by the caller),
 // followed by launch_fold into prm.gvol.
