@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(256, 6) k_spectral_from_L(const MarchParams pr
 enum { kEach, kMerge, kDirect };
 template <int M, int MODE, bool FROM_GL, int KIND>
 __global__ void __launch_bounds__(256, 4)
-    k_backward(const MarchParams prm, int tile_u, int warp_rows, int tiles_v, int group0)
+    k_backward(const MarchParams prm, int tile_u, int warp_rows, int tiles_v, int group0, bool parts_in_y)
 {
     extern __shared__ __align__(16) float s_mu[];
     if (!FROM_GL) load_mu(s_mu, prm.mu, prm.E, M);
@@ -412,18 +412,20 @@ __global__ void __launch_bounds__(256, 4)
     const int tile_v = (int)blockDim.x / tile_u;
     const int wcols = 32 / warp_rows, warps_u = tile_u / wcols;
     const int u = blockIdx.x * tile_u + (w % warps_u) * wcols + lane / warp_rows;
-    const int part = blockIdx.z / tiles_v, band = blockIdx.z % tiles_v;
+    // the parts of the views: z, or interleaved in y (parts_in_y)
+    const int parts = prm.sets / prm.set_columns;
+    const int part = parts_in_y ? blockIdx.y % parts : blockIdx.z / tiles_v;
+    const int group = group0 + (int)(parts_in_y ? blockIdx.y / parts : blockIdx.y), band = parts_in_y ? blockIdx.z : blockIdx.z % tiles_v;
     const int v = band * tile_v + (w / warps_u) * warp_rows + lane % warp_rows;
     const bool ray_on = u < prm.g.U && v < prm.g.V;
     const int64_t npix = (int64_t)prm.g.U * prm.g.V;
     const int64_t pix = (int64_t)v * prm.g.U + u;
     // the part's views, each part's as many as another's or one more
-    const int parts = prm.sets / prm.set_columns;
     const int first = prm.view0 + (int)((int64_t)prm.n_views * part / parts);
     const int pend = prm.view0 + (int)((int64_t)prm.n_views * (part + 1) / parts);
     const int set = part * prm.set_columns + (u & (prm.set_columns - 1));
     for (int k = 0; k < prm.views_per_cta; k++) {
-        const int p = first + (group0 + blockIdx.y) * prm.views_per_cta + k;
+        const int p = first + group * prm.views_per_cta + k;
         if (p >= pend) break;
         const int64_t ray = (int64_t)(p - prm.out_view0) * npix + pix;
         float g[M];
@@ -1092,21 +1094,27 @@ cudaError_t axis_dispatch(const MarchParams& prm, int interp, bool spec, int min
 
 // Whether the scatter of three or four materials hands sums over between rows
 // (flush_voxels): the shuffles pay while neighbouring rows mostly flush
-// neighbouring voxels, and for the texture emulation, whose samples cost more
-// instructions, only where the L2's reductions bind.  Measured, adjoint + fold,
-// each lane on its own / merged, ms -- trilinear, 3 materials: 64^3, row
-// spacing 1.3 voxels 0.392 / 0.346, 176^3, 1.0 5.69 / 4.37, 128^3, 2.0 1.00 / 1.08;
-// texture emulation: 96^3, 1.0 1.03 / 1.06, 128^3, 0.5 3.76 / 3.22, 256^3, 1.3
-// 9.47 / 8.66, 128^3, 2.0 1.03 / 1.13.
-bool merge_faces(const GeomParams& g, int interp)
+// neighbouring voxels (spacing), there are neighbours in a warp (rows), and the
+// L2's reductions bind rather than a ray's own chain: from a full chip of rays
+// on, and for the texture emulation, whose samples cost more instructions, where
+// the accumulators are large or the rays dense.  Measured, adjoint + fold, each
+// lane on its own / merged, ms -- trilinear, 3 materials: 64^3, row spacing 1.3
+// voxels 0.392 / 0.346, 176^3, 1.0 5.69 / 4.37, 128^3, 2.0 1.00 / 1.08; 96 x 96 x
+// 16, 180 views of 1 / 2 / 3 / 5 / 8 / 13 rows 0.19 / 0.29, 0.20 / 0.30, 0.28 / 0.35,
+// 0.36 / 0.43, 0.55 / 0.46, 0.67 / 0.53; 32^3, 46 k rays 0.085 / 0.103; texture emulation: 96^3, 1.0
+// 1.03 / 1.06, 0.8 (180 views) 4.63 / 3.77, 128^3, 0.5 3.76 / 3.22, 256^3, 1.3 9.47 /
+// 8.66, 128^3, 2.0 1.03 / 1.13, 96 x 96 x 16, 8 rows 0.8 0.59 / 0.51.
+bool merge_faces(const MarchParams& prm, int interp)
 {
+    const GeomParams& g = prm.g;
     const float rows = g.dSize * g.sod / (g.sdd * g.pSizeZ);
-    if (rows >= 1.8f) return false;
-    return interp == INTERP_TRILINEAR || rows < 0.7f || (int64_t)g.nx * g.ny * g.nz > 2000000;
+    if (rows >= 1.8f || g.V < 8 || (int64_t)prm.n_views * g.U * g.V < 150000) return false;
+    return interp == INTERP_TRILINEAR || rows < 0.9f || (int64_t)g.nx * g.ny * g.nz > 2000000;
 }
 
 struct BwdGrid {
     int tile_u, rows, tiles_v, group0;
+    bool parts_in_y;
     dim3 grid, block;
     size_t smem;
 };
@@ -1117,8 +1125,8 @@ cudaError_t bwd_launch(const MarchParams& prm, const BwdGrid& b, cudaStream_t st
     const size_t smem = FROM_GL ? 0 : b.smem;
     auto k = k_backward<M, MODE, FROM_GL, kEach>;
     if (!prm.gcol) k = k_backward<M, MODE, FROM_GL, kDirect>;
-    else if (M > 2 && merge_faces(prm.g, MODE)) k = k_backward<M, MODE, FROM_GL, (M > 2 ? kMerge : kEach)>;
-    k<<<b.grid, b.block, smem, st>>>(prm, b.tile_u, b.rows, b.tiles_v, b.group0);
+    else if (M > 2 && merge_faces(prm, MODE)) k = k_backward<M, MODE, FROM_GL, (M > 2 ? kMerge : kEach)>;
+    k<<<b.grid, b.block, smem, st>>>(prm, b.tile_u, b.rows, b.tiles_v, b.group0, b.parts_in_y);
     return cudaGetLastError();
 }
 
@@ -1376,9 +1384,11 @@ cudaError_t launch_backward(const MarchParams& prm_in, int M, int interp, bool f
     // fold of 24 views of 128^3, row spacing in voxels: 8 / 16 / 32 rows, ms --
     // 1 material 0.25: 4.72 / 3.78 / 3.75, 0.6: 1.05 / 1.02 / 1.09, 1.05: 0.46 /
     // 0.47 / 0.49; 3 materials 0.25: 11.96 / 10.07 / 9.17, 1.05: 0.86 / 0.84 / 0.88.
+    // A detector of fewer rows: no more than hold them all (one row, 96 x 96 x 16, 180
+    // views, 4 rows / 1, 1 material 0.167 / 0.131, 3 materials 0.345 / 0.192).
     const GeomParams& g = prm_in.g;
     int rows = g.dSize * g.sod < 0.35f * g.sdd * g.pSizeZ ? 32 : 16;
-    while (rows > 4 && rows / 2 >= g.V) rows /= 2;
+    while (rows > 1 && rows / 2 >= g.V) rows /= 2;
     const int threads = ls.tile_u * ls.tile_v;
     LaunchShape bs = ls;
     if (bs.tile_v % rows != 0 || bs.tile_u % (32 / rows) != 0) {
@@ -1398,8 +1408,14 @@ cudaError_t launch_backward(const MarchParams& prm_in, int M, int interp, bool f
     const int parts = prm.sets / prm.set_columns, views = (prm.n_views + parts - 1) / parts;  // of the largest part
     prm.views_per_cta = std::max(1, std::min(ls.views_per_cta, views));
     const int groups = (views + prm.views_per_cta - 1) / prm.views_per_cta;
-    for (b.group0 = 0; b.group0 < groups; b.group0 += 65535) {
-        b.grid = dim3(tiles_u, std::min(65535, groups - b.group0), b.tiles_v * parts);
+    // One band of rows and elements of 16 bytes: the parts at the same time, since the
+    // CTAs of neighbouring views reduce into the same few voxels (8 rows, 3 materials
+    // 0.457 -> 0.424 ms, 5 rows 0.357 -> 0.334; pair cells lose, 1 material, 2 rows 0.125 -> 0.135).
+    b.parts_in_y = M > 2 && b.tiles_v == 1;
+    const int most = b.parts_in_y ? 65535 / parts : 65535;
+    for (b.group0 = 0; b.group0 < groups; b.group0 += most) {
+        const int n = std::min(most, groups - b.group0);
+        b.grid = b.parts_in_y ? dim3(tiles_u, n * parts, 1) : dim3(tiles_u, n, b.tiles_v * parts);
         if (b.grid.x == 0 || b.grid.y == 0 || b.grid.z == 0) return cudaSuccess;
         cudaError_t e = cudaErrorInvalidValue;
         switch (M) {
