@@ -216,7 +216,7 @@ __device__ __forceinline__ void batch_march(const ItemDesc& it, const ItemTex<M>
 // dLoss/dL it takes from shared memory.  4 items of 96^3, 3 materials, forward + loss +
 // adjoint, both down the rows / both along the columns / exchanged: z-layered
 // 4.89 / 3.38 / 3.03 ms, hardware texture 3.42 / 3.79 / 2.82.
-template <int M, int MODE, bool ADJOINT, bool AXIS>
+template <int M, int MODE, bool ADJOINT, bool AXIS, bool MERGE>
 __device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M>& tx, const float* s_mu, float (*s_g)[64],
                                              int set, int p, int u0, int v0, int du, int dv, int tile_v)
 {
@@ -281,7 +281,7 @@ __device__ __forceinline__ float process_ray(const ItemDesc& it, const ItemTex<M
     if (!AXIS && !it.gcol) scatter_direct<M, SM>(it.g, it.gvol, any, p, v, u, g);
     else {
         const int cols = it.sets / it.set_parts, at = set * cols + (u & (cols - 1));
-        scatter_columns<M, SM, (M > 2 && MODE == INTERP_TRILINEAR)>(it.g, it.gcol + (size_t)at * it.set_floats, any, p, v, u, g);
+        scatter_columns<M, SM, MERGE>(it.g, it.gcol + (size_t)at * it.set_floats, any, p, v, u, g);
     }
     return res * res;
 }
@@ -308,7 +308,7 @@ struct BatchBudget {
 // MULTI: units of more than one view (a.vpu > 1), marched one view after the
 // other; the one-view kernel has no view loop, whose live state cost the fused
 // axis kernel 3 % on the 48-problem batch.
-template <int M, int MODE, bool ADJOINT, bool AXIS, bool MULTI>
+template <int M, int MODE, bool ADJOINT, bool AXIS, bool MULTI, bool MERGE>
 __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJOINT, M, MODE, AXIS>::minb)
     k_batch(const GroupArgs a)
 {
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(BatchShape<ADJOINT>::threads, BatchBudget<ADJO
             }
             const int pk = *(volatile int*)&s_p * (MULTI ? a.vpu : 1) + k;
             if (pk >= it.g.P) break;
-            loss += process_ray<M, MODE, ADJOINT, AXIS>(it, tx, s_mu, s_g, ADJOINT ? s_set : 0, pk, *(volatile int*)&s_tu * tile_u,
+            loss += process_ray<M, MODE, ADJOINT, AXIS, MERGE>(it, tx, s_mu, s_g, ADJOINT ? s_set : 0, pk, *(volatile int*)&s_tu * tile_u,
                                                         *(volatile int*)&s_tv * tile_v, du, dv, tile_v);
         }
         if (ADJOINT) {
@@ -443,34 +443,49 @@ __global__ void __launch_bounds__(256) k_batch_fold(const ItemDesc* items, int n
 
 using KernelFn = void (*)(GroupArgs);
 
-template <int M, bool ADJOINT, bool MULTI>
-KernelFn kernel_for_m(int interp, bool axis)
+// Whether an item's scatter hands sums over between rows (flush_voxels;
+// merge_faces of the plan's adjoint says why): groups of their own.  4 items of
+// 96^3, 3 materials, forward + loss + adjoint, never / always, ms: rows 0.7 voxels apart
+// 4.94 / 4.84, 2.0 1.12 / 1.15, 3.0 0.77 / 0.80; one row 1.27 / 1.52.
+bool merges(int M, int interp, const GeomParams& g)
 {
+    return M > 2 && interp == INTERP_TRILINEAR && g.V >= 8 && g.dSize * g.sod < 1.8f * g.sdd * g.pSizeZ;
+}
+
+template <int M, bool ADJOINT, bool MULTI>
+KernelFn kernel_for_m(int interp, bool axis, bool merge)
+{
+    constexpr bool can = ADJOINT && M > 2;
+    if (interp == INTERP_TRILINEAR && merge)
+        return axis ? k_batch<M, INTERP_TRILINEAR, ADJOINT, true, MULTI, can>
+                    : k_batch<M, INTERP_TRILINEAR, ADJOINT, false, MULTI, can>;
     if (interp == INTERP_TRILINEAR)
-        return axis ? k_batch<M, INTERP_TRILINEAR, ADJOINT, true, MULTI>
-                    : k_batch<M, INTERP_TRILINEAR, ADJOINT, false, MULTI>;
+        return axis ? k_batch<M, INTERP_TRILINEAR, ADJOINT, true, MULTI, false>
+                    : k_batch<M, INTERP_TRILINEAR, ADJOINT, false, MULTI, false>;
     if (interp == INTERP_TEXEMU)
-        return axis ? k_batch<M, INTERP_TEXEMU, ADJOINT, true, MULTI> : k_batch<M, INTERP_TEXEMU, ADJOINT, false, MULTI>;
-    return k_batch<M, INTERP_TEXTURE, ADJOINT, false, MULTI>;
+        return axis ? k_batch<M, INTERP_TEXEMU, ADJOINT, true, MULTI, false>
+                    : k_batch<M, INTERP_TEXEMU, ADJOINT, false, MULTI, false>;
+    return k_batch<M, INTERP_TEXTURE, ADJOINT, false, MULTI, false>;
 }
 
 template <bool ADJOINT, bool MULTI>
-KernelFn kernel_for_v(int M, int interp, bool axis)
+KernelFn kernel_for_v(int M, int interp, bool axis, bool merge)
 {
     switch (M) {
-        case 1: return kernel_for_m<1, ADJOINT, MULTI>(interp, axis);
-        case 2: return kernel_for_m<2, ADJOINT, MULTI>(interp, axis);
-        case 3: return kernel_for_m<3, ADJOINT, MULTI>(interp, axis);
-        default: return kernel_for_m<4, ADJOINT, MULTI>(interp, axis);
+        case 1: return kernel_for_m<1, ADJOINT, MULTI>(interp, axis, merge);
+        case 2: return kernel_for_m<2, ADJOINT, MULTI>(interp, axis, merge);
+        case 3: return kernel_for_m<3, ADJOINT, MULTI>(interp, axis, merge);
+        default: return kernel_for_m<4, ADJOINT, MULTI>(interp, axis, merge);
     }
 }
 
 // The kernel of one kind of call for units of vpu views (both variants have
 // the same register budget, hence the same persistent grid).
 template <bool ADJOINT>
-KernelFn kernel_for(int M, int interp, bool axis, int vpu = 1)
+KernelFn kernel_for(int M, int interp, bool axis, bool merge, int vpu = 1)
 {
-    return vpu > 1 ? kernel_for_v<ADJOINT, true>(M, interp, axis) : kernel_for_v<ADJOINT, false>(M, interp, axis);
+    return vpu > 1 ? kernel_for_v<ADJOINT, true>(M, interp, axis, merge)
+                   : kernel_for_v<ADJOINT, false>(M, interp, axis, merge);
 }
 
 }  // namespace
@@ -490,7 +505,7 @@ struct ctfp_batch {
     std::vector<long long> tile0;      // first block of each slot in the fold's grid
     std::vector<ItemDesc> items;       // tables of the current call
     struct Group {
-        int M, interp, axis, first, count;
+        int M, interp, axis, merge, first, count;
         long long begin, end;
         int grid[2];                   // persistent grid: forward, forward + adjoint
     };
@@ -557,8 +572,8 @@ ctfp_status record(ctfp_batch* b, bool adjoint, const std::vector<const float*>&
         GroupArgs a{table, G.first, G.count, G.begin, end, b->d_counter + gi,
                     __builtin_ctz((unsigned)b->tile_u[adjoint ? 1 : 0]), b->vpu[adjoint ? 1 : 0]};
         const int vpu = b->vpu[adjoint ? 1 : 0];
-        KernelFn fn = adjoint ? kernel_for<true>(G.M, G.interp, G.axis, vpu)
-                              : kernel_for<false>(G.M, G.interp, G.axis, vpu);
+        KernelFn fn = adjoint ? kernel_for<true>(G.M, G.interp, G.axis, G.merge, vpu)
+                              : kernel_for<false>(G.M, G.interp, G.axis, G.merge, vpu);
         fn<<<G.grid[adjoint ? 1 : 0], kind_threads(adjoint ? 1 : 0), 0, st>>>(a);
         BATCH_CUDA(cudaGetLastError());
     }
@@ -724,7 +739,7 @@ ctfp_status ctfp_batch_create(int32_t n_items, ctfp_plan* const* plans, ctfp_bat
     b->n = n_items;
     b->device = dev;
     b->plans.assign(plans, plans + n_items);
-    // group by (materials, mode), groups by total cost; within a group cost
+    // group by (materials, mode, hand-over), groups by total cost; within a group cost
     // order (rays x samples x materials), largest first: the queue hands out
     // units in this order (longest-processing-time-first list scheduling)
     std::vector<double> cost((size_t)n_items);
@@ -733,9 +748,10 @@ ctfp_status ctfp_batch_create(int32_t n_items, ctfp_plan* const* plans, ctfp_bat
         cost[(size_t)i] = (double)g.U * g.V * g.P * g.K * plan_materials(plans[i]);
     }
     auto gkey = [&](int i) {
-        return (plan_materials(plans[i]) * 4 + plan_interp(plans[i])) * 2 + (uses_axis(plans[i]) ? 1 : 0);
+        const int mode = (plan_materials(plans[i]) * 4 + plan_interp(plans[i])) * 2 + (uses_axis(plans[i]) ? 1 : 0);
+        return mode * 2 + (merges(plan_materials(plans[i]), plan_interp(plans[i]), plan_geom(plans[i])) ? 1 : 0);
     };
-    std::vector<double> gcost(64, 0.0);
+    std::vector<double> gcost(128, 0.0);
     for (int i = 0; i < n_items; i++) gcost[(size_t)gkey(i)] += cost[(size_t)i];
     b->order.resize((size_t)n_items);
     std::iota(b->order.begin(), b->order.end(), 0);
@@ -755,11 +771,11 @@ ctfp_status ctfp_batch_create(int32_t n_items, ctfp_plan* const* plans, ctfp_bat
         ItemDesc& it = b->items[(size_t)s];
         it.M = plan_materials(p);
         it.interp = plan_interp(p);
-        const int ax = uses_axis(p) ? 1 : 0;
+        const int ax = uses_axis(p) ? 1 : 0, merge = merges(it.M, it.interp, g) ? 1 : 0;
         b->item_axis[(size_t)s] = ax != 0;
         if (b->groups.empty() || b->groups.back().M != it.M || b->groups.back().interp != it.interp ||
-            b->groups.back().axis != ax)
-            b->groups.push_back({it.M, it.interp, ax, s, 0, unit, unit, {0, 0}});
+            b->groups.back().axis != ax || b->groups.back().merge != merge)
+            b->groups.push_back({it.M, it.interp, ax, merge, s, 0, unit, unit, {0, 0}});
         b->groups.back().count++;
         b->tile0[(size_t)s] = tiles;
         tiles += column_tiles(g.nx, g.ny, g.nz);
@@ -797,7 +813,7 @@ ctfp_status ctfp_batch_create(int32_t n_items, ctfp_plan* const* plans, ctfp_bat
     for (ctfp_batch::Group& G : b->groups) {
         for (int k = 0; k < 2 && e == cudaSuccess; k++) {
             int per = 0;
-            KernelFn fn = k ? kernel_for<true>(G.M, G.interp, G.axis) : kernel_for<false>(G.M, G.interp, G.axis);
+            KernelFn fn = k ? kernel_for<true>(G.M, G.interp, G.axis, G.merge) : kernel_for<false>(G.M, G.interp, G.axis, G.merge);
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kind_threads(k), 0);
             G.grid[k] = std::max(1, per) * std::max(1, nsm);
         }
