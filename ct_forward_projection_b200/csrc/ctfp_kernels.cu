@@ -200,17 +200,18 @@ __global__ void __launch_bounds__(256, MINB) k_forward_axis(const MarchParams pr
 // K1+K2 with the axis sampler for a plan of few rays (axis_split), where a
 // thread per ray leaves most of the chip idle and the time is one ray's chain
 // of gathers: 1 << shift lanes share a ray, each marching an equal run of its
-// samples and taking a fourth of the energies.  A warp covers 32 >> shift rows
-// of one column (lane quads down 4 rows, as k_forward_axis), a CTA 4 columns.
+// samples and taking a fourth of the energies.  A warp covers 32 >> shift rays,
+// rows of a column (lane quads down 4 rows, as k_forward_axis) or, where the
+// detector has fewer rows, that many rows of several columns; a CTA 4 warps.
 // The energies' partial sums are spectral()'s four accumulators, combined in
 // its order, so I and IAbs equal its values for the same L.
 template <int M, int MODE, bool SKIP, bool SPECTRAL>
-__global__ void __launch_bounds__(128, uses_columns(M) ? 6 : 8) k_forward_axis_split(const MarchParams prm, int shift)
+__global__ void __launch_bounds__(128, uses_columns(M) ? 6 : 8) k_forward_axis_split(const MarchParams prm, int shift, int rows)
 {
     extern __shared__ __align__(16) float s_mu[];
     if (SPECTRAL) load_mu(s_mu, prm.mu, prm.E, M);
-    const int lane = threadIdx.x & 31, rows = 32 >> shift, part = lane / rows;
-    const int u = blockIdx.x * 4 + (threadIdx.x >> 5), v = blockIdx.y * rows + lane % rows;
+    const int lane = threadIdx.x & 31, rays = 32 >> shift, part = lane / rays, ray_at = lane % rays, cols = rays / rows;
+    const int u = (blockIdx.x * 4 + (threadIdx.x >> 5)) * cols + ray_at / rows, v = blockIdx.y * rows + ray_at % rows;
     const int p = prm.view0 + blockIdx.z;
     const bool on = u < prm.g.U && v < prm.g.V;
     const int64_t npix = (int64_t)prm.g.U * prm.g.V;
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(128, uses_columns(M) ? 6 : 8) k_forward_axis_s
         const OccView ov{prm.occ, prm.occ_x, prm.occ_y, prm.g.nx, prm.g.ny, prm.g.nz, kOccShift};
         march_axis_sums<M, MODE, SKIP>(prm.g, prm.xtex, prm.ytex, prm.cvol, ov, p, v, u, L, cmp, part, 1 << shift);
     }
-    for (int d = rows; d < 32; d <<= 1)
+    for (int d = rays; d < 32; d <<= 1)
 #pragma unroll
         for (int m = 0; m < M; m++)
             kahan_join(L[m], cmp[m], __shfl_xor_sync(0xffffffffu, L[m], d), __shfl_xor_sync(0xffffffffu, cmp[m], d));
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(128, uses_columns(M) ? 6 : 8) k_forward_axis_s
                 sA += tA;
             }
         }
-        for (int d = rows; d < 4 * rows / own; d <<= 1) {
+        for (int d = rays; d < 4 * rays / own; d <<= 1) {
             sI += __shfl_xor_sync(0xffffffffu, sI, d);
             sA += __shfl_xor_sync(0xffffffffu, sA, d);
         }
@@ -1150,11 +1151,15 @@ template <int M, int MODE, bool SKIP>
 cudaError_t split_launch(const MarchParams& prm, bool spec, int shift, cudaStream_t st)
 {
     const size_t smem = spec ? sizeof(float) * (size_t)energy_groups(prm.E) * 4 * M : 0;
-    const int rows = 32 >> shift;
-    const dim3 grid((prm.g.U + 3) / 4, (prm.g.V + rows - 1) / rows, prm.n_views);
+    // no more rows than the detector has (one row of 400 pixels, 360 views of 128^2,
+    // 4 lanes a ray, 8 rows / 1: 830 / 168 us)
+    int rows = 32 >> shift;
+    while (rows > 1 && rows / 2 >= prm.g.V) rows /= 2;
+    const int cols = 4 * (32 >> shift) / rows;  // of a CTA
+    const dim3 grid((prm.g.U + cols - 1) / cols, (prm.g.V + rows - 1) / rows, prm.n_views);
     if (grid.x == 0 || grid.y == 0 || grid.z == 0) return cudaSuccess;
-    if (spec) k_forward_axis_split<M, MODE, SKIP, true><<<grid, 128, smem, st>>>(prm, shift);
-    else k_forward_axis_split<M, MODE, SKIP, false><<<grid, 128, smem, st>>>(prm, shift);
+    if (spec) k_forward_axis_split<M, MODE, SKIP, true><<<grid, 128, smem, st>>>(prm, shift, rows);
+    else k_forward_axis_split<M, MODE, SKIP, false><<<grid, 128, smem, st>>>(prm, shift, rows);
     return cudaGetLastError();
 }
 
