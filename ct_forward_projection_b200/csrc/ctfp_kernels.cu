@@ -1132,19 +1132,26 @@ cudaError_t bwd_launch(const MarchParams& prm, const BwdGrid& b, cudaStream_t st
 }
 
 // log2 of the lanes per ray of a plan's march: 0 is k_forward_axis, one thread
-// per ray.  It depends on the plan's rays alone, so that every call of a plan
-// (a range of its views, any launch shape) sums a ray the same way.  The chip
-// holds 150 k threads of the march at a time: below a few times that, a thread
-// per ray runs as long as its longest ray plus a nearly empty last wave.
-// Measured, us a forward with 1 / 2 / 4 / 8 lanes per ray (2 materials unless
-// noted): 15 k rays of 32^3 57 / - / 44 / 43, 16 k of 64^3 103 / - / 43 / 38, 66 k
-// of 128^3 221 / - / 99 / 97, 144 k of 96^3 191 / - / 128 / 141, 393 k of 128^3
-// 367 / - / 308 / 346, 655 k of 128^3 531 / 453 / 473, 819 k of 64^3 365 / 398 /
-// 386, 1.0 M of 128^3 743 / 694 / 732 and (128 rows more) 690 / 678 / 697.
-int axis_split(const GeomParams& g)
+// per ray.  It depends on the plan alone, so that every call of it (a range of its
+// views, any launch shape) sums a ray the same way.  The chip holds 148 x 1024
+// threads of the march at a time (148 x 768 of four materials'): while the rays
+// leave it part empty, the time is one ray's chain of gathers, and as many lanes
+// share a ray as fit.  Past that 2 lanes still pay, by a shorter last wave, the
+// longer the rays are: up to some 5500 rays for each voxel of nx + ny (2 samples a
+// voxel; where empty space is skipped, half of them).  Measured, us a forward with 1
+// / 2 / 4 / 8 lanes per ray, 2 materials -- 18 k rays of 32^3 50 / 29 / 28 / 28, 64^3 89 /
+// 46 / 31 / 31, 128^3 204 / 90 / 67 / 56 (4 materials 183 / 68 / 49 / 63), 256^3 769 / 352 /
+// 269 / 233; 55 k of 32^3 48 / 31 / 35 / 44, 128^3 199 / 91 / 99 / 99; 197 k of 32^3 77 / 72 /
+// 85 / 117, 128^3 272 / 219 / 220 / 249; 390 k of 32^3 124 / 126 / 152 / 218, 64^3 220 / 202 /
+// 228 / 295, 256^3 1303 / 1039 / 1098 / 1221; 688 k of 32^3 197 / 210 / 258 / 376, 64^3 349 /
+// 340 / 389 / 510 (half of it empty and skipped 356 / 379), 128^3 691 / 631 / 659 / 771;
+// 897 k of 64^3 440 / 434, 128^3 849 / 804, 256^3 2189 / 2135, 3 and 4 materials 3789 / 3940, 3272 / 3656.
+int axis_split(const GeomParams& g, int M, bool skip)
 {
-    const int64_t rays = (int64_t)g.U * g.V * g.P;
-    return rays <= 20000 ? 3 : rays <= 400000 ? 2 : rays <= 700000 ? 1 : 0;
+    const int64_t rays = (int64_t)g.U * g.V * g.P, chip = 148 * (uses_columns(M) ? 768 : 1024);
+    const int64_t voxels = (int64_t)(g.nx + g.ny) >> (skip ? 1 : 0);
+    if (rays > std::max<int64_t>(chip, std::min<int64_t>(700000, 5500 * voxels))) return 0;
+    return 8 * rays <= chip ? 3 : 4 * rays <= chip ? 2 : 1;
 }
 
 template <int M, int MODE, bool SKIP>
@@ -1214,8 +1221,8 @@ cudaError_t launch_forward_once(const MarchParams& prm, int M, int interp, int s
         }
         return cudaErrorInvalidValue;
     }
-    if (sampler == SAMPLER_AXIS && interp != INTERP_TEXTURE && axis_split(prm.g) > 0) {
-        const int shift = axis_split(prm.g);
+    if (sampler == SAMPLER_AXIS && interp != INTERP_TEXTURE && axis_split(prm.g, M, prm.occ) > 0) {
+        const int shift = axis_split(prm.g, M, prm.occ);
         switch (M) {
             case 1: return split_dispatch<1>(prm, interp, do_spectral, shift, st);
             case 2: return split_dispatch<2>(prm, interp, do_spectral, shift, st);
@@ -1263,7 +1270,7 @@ cudaError_t launch_forward(const MarchParams& prm_in, int M, int interp, int sam
                            const LaunchShape& ls, cudaStream_t st)
 {
     // view groups run along grid.z, at most 65535 per launch
-    const bool split = sampler == SAMPLER_AXIS && interp != INTERP_TEXTURE && axis_split(prm_in.g) > 0;
+    const bool split = sampler == SAMPLER_AXIS && interp != INTERP_TEXTURE && axis_split(prm_in.g, M, prm_in.occ) > 0;
     const int vpc = split ? 1 : ls.views_per_cta;
     const int max_views = 65535 * vpc;
     for (int v0 = 0; v0 < prm_in.n_views; v0 += max_views) {
