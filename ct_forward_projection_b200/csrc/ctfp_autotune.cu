@@ -12,7 +12,9 @@
 // per process under a key of the geometry, materials, sampler, energies and
 // device name, and optionally in
 // the text file named by CTFP_TUNE_CACHE (one "key tile_u tile_v views
-// min_ctas ms" line per entry), which later processes read.
+// min_ctas ms" line per entry), which later processes read.  A plan whose rays
+// are shared by lanes (axis_split) marches in one shape only: it is timed and
+// the plan's shape, which its adjoint uses, stays as it is.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -59,7 +61,9 @@ ctfp_status tfail(ctfp_status st, const std::string& m)
     return st;
 }
 
-std::string cache_key(const ctfp_plan* p, int n_sample)
+// An entry counts for the kernel it was timed with: four materials over the
+// column copy, and plans whose forward has no shape to choose, have their own.
+std::string cache_key(const ctfp_plan* p, int n_sample, bool fixed)
 {
     const ctfp_geometry& g = plan_geometry(p);
     cudaDeviceProp prop;
@@ -72,6 +76,9 @@ std::string cache_key(const ctfp_plan* p, int n_sample)
       << g.pLengthZ << "|P" << g.projNum << "|" << g.dNumU << "x" << g.dNumV << "@" << g.dSize << "|" << g.sod << ","
       << g.sdd << "|M" << plan_materials(p) << "|i" << plan_interp(p) << "|s" << plan_sampler(p) << "|E"
       << plan_energies(p) << "|n" << n_sample;
+    if (plan_sampler(p) == SAMPLER_AXIS && plan_interp(p) != INTERP_TEXTURE && axis_uses_columns(plan_materials(p)))
+        k << "|columns";
+    if (fixed) k << "|split";
     return k.str();
 }
 
@@ -179,18 +186,20 @@ extern "C" ctfp_status ctfp_plan_autotune(ctfp_plan* p, const float* const* volu
     const GeomParams& g = plan_geom(p);
     int n = n_sample_views > 0 ? n_sample_views : 64;
     n = std::min(n, g.P);
-    const std::string key = cache_key(p, n);
+    // rays shared by lanes: the launch shape is the adjoint's alone, and stays
+    const bool fixed = forward_splits(plan_march_params(p), plan_materials(p), plan_interp(p), plan_sampler(p));
+    const std::string key = cache_key(p, n, fixed);
     {
         std::lock_guard<std::mutex> lk(g_mu);
         read_file_cache();
         auto it = g_cache.find(key);
         if (it != g_cache.end() && valid_shape(it->second.shape)) {
-            plan_shape(p) = it->second.shape;
+            if (!fixed) plan_shape(p) = it->second.shape;
             if (out) {
-                out->tile_u = it->second.shape.tile_u;
-                out->tile_v = it->second.shape.tile_v;
-                out->views_per_cta = it->second.shape.views_per_cta;
-                out->min_ctas_per_sm = it->second.shape.min_ctas;
+                out->tile_u = plan_shape(p).tile_u;
+                out->tile_v = plan_shape(p).tile_v;
+                out->views_per_cta = plan_shape(p).views_per_cta;
+                out->min_ctas_per_sm = plan_shape(p).min_ctas;
                 out->ms = it->second.ms;
                 out->from_cache = 1;
             }
@@ -221,7 +230,11 @@ extern "C" ctfp_status ctfp_plan_autotune(ctfp_plan* p, const float* const* volu
     if (rs == CTFP_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess ||
                           cs.create() != cudaSuccess))
         rs = tfail(CTFP_CUDA_ERROR, "cudaEventCreate / cudaStreamCreate failed");
-    if (rs == CTFP_OK) {
+    if (rs == CTFP_OK && fixed) {
+        best.ms = time_shape(base, M, interp, sampler, best.shape, chunks, e0, e1, st, cs, 2);
+        if (best.ms < 0.f)
+            rs = tfail(CTFP_CUDA_ERROR, std::string("autotune launch: ") + cudaGetErrorString(cudaGetLastError()));
+    } else if (rs == CTFP_OK) {
         static const int tiles[][2] = {{16, 8}, {32, 4}, {8, 16}, {64, 2}, {16, 16}, {32, 8}, {8, 32}, {64, 4},
                                        {8, 8},  {16, 4}};
         std::vector<Entry> stage1;

@@ -1221,7 +1221,7 @@ cudaError_t launch_forward_once(const MarchParams& prm, int M, int interp, int s
         }
         return cudaErrorInvalidValue;
     }
-    if (sampler == SAMPLER_AXIS && interp != INTERP_TEXTURE && axis_split(prm.g, M, prm.occ) > 0) {
+    if (forward_splits(prm, M, interp, sampler)) {
         const int shift = axis_split(prm.g, M, prm.occ);
         switch (M) {
             case 1: return split_dispatch<1>(prm, interp, do_spectral, shift, st);
@@ -1266,12 +1266,16 @@ cudaError_t launch_forward_once(const MarchParams& prm, int M, int interp, int s
 
 }  // namespace
 
+bool forward_splits(const MarchParams& prm, int M, int interp, int sampler)
+{
+    return sampler == SAMPLER_AXIS && interp != INTERP_TEXTURE && axis_split(prm.g, M, prm.occ) > 0;
+}
+
 cudaError_t launch_forward(const MarchParams& prm_in, int M, int interp, int sampler, bool do_spectral,
                            const LaunchShape& ls, cudaStream_t st)
 {
     // view groups run along grid.z, at most 65535 per launch
-    const bool split = sampler == SAMPLER_AXIS && interp != INTERP_TEXTURE && axis_split(prm_in.g, M, prm_in.occ) > 0;
-    const int vpc = split ? 1 : ls.views_per_cta;
+    const int vpc = forward_splits(prm_in, M, interp, sampler) ? 1 : ls.views_per_cta;
     const int max_views = 65535 * vpc;
     for (int v0 = 0; v0 < prm_in.n_views; v0 += max_views) {
         MarchParams prm = prm_in;

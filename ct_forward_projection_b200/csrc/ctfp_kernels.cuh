@@ -63,6 +63,8 @@ struct LaunchShape {
 cudaError_t launch_forward(const MarchParams& prm, int M, int interp, int sampler, bool do_spectral,
                            const LaunchShape& ls, cudaStream_t st);
 cudaError_t launch_spectral_from_L(const MarchParams& prm, int M, cudaStream_t st);
+// Whether this forward shares rays among lanes (axis_split), in its own launch shape.
+bool forward_splits(const MarchParams& prm, int M, int interp, int sampler);
 // Floats of one set of the adjoint's accumulators (accum_width).
 size_t accum_floats(int nx, int ny, int nz, int M);
 int accum_set_count(const GeomParams& g, int n_views, int M);  // accum_sets, any number of sets

@@ -105,7 +105,7 @@ typedef enum ctfp_sampler {
      * fetched.  Results agree with the layered sampler to FP32 rounding (the
      * layer axis is interpolated last).  Plans of four materials hold one
      * z-fastest copy instead, the four materials of a voxel side by side, and
-     * load the missing corners from it; plans of at most 700 000 rays march a
+     * load the missing corners from it; plans of few rays march a
      * ray with 2, 4 or 8 threads.  The default; needs pNumX, pNumY <= 2046
      * and pNumZ <= 32768 (else the layered sampler, else the global one). */
     CTFP_SAMPLER_AXIS = 4
@@ -146,7 +146,10 @@ ctfp_status ctfp_plan_set_sampler(ctfp_plan* plan, int32_t sampler);
  * CTA for its tile, and min_ctas_per_sm (2, 3, 4, or 5 for the axis sampler;
  * other samplers run 5 as 4), the residency the forward march is compiled for
  * (its register cap: 65536 / (256 * min_ctas_per_sm)).
- * Set by the autotuner; defaults 16 x 8 x 2 x 4. */
+ * Set by the autotuner; defaults 16 x 8 x 2 x 4, of four materials 16 x 8 x 2 x
+ * 3.  The forward of a plan of at most 700 000 rays through the axis sampler may
+ * share each ray among lanes, in a shape of its own; the plan's is then the
+ * adjoint's alone. */
 ctfp_status ctfp_plan_set_launch_shape(ctfp_plan* plan, int32_t tile_u, int32_t tile_v, int32_t views_per_cta,
                                        int32_t min_ctas_per_sm);
 
@@ -299,7 +302,8 @@ ctfp_status ctfp_check_division(int32_t device, float divisor, int64_t n, uint64
  * all 360 pick (2 views per CTA), 16 pick 1 view per CTA, 5 % slower on the
  * whole forward.  Tuning takes about 36 forwards of the sample.  I and IAbsorb
  * are full-size output buffers as for ctfp_forward; their contents are
- * undefined afterwards.  Synchronises the stream.  Results are cached per
+ * undefined afterwards.  A forward that shares rays among lanes has one shape:
+ * it is timed, and the plan's shape stays.  Synchronises the stream.  Results are cached per
  * process by geometry, materials, sampler, energies and device name, and in the
  * text file named by the environment variable CTFP_TUNE_CACHE when it is set. */
 typedef struct ctfp_launch_shape {
@@ -506,7 +510,8 @@ ctfp_status ctfp_count_support_samples(ctfp_plan* plan, int64_t* out);
  * (as the layered sampler's two gathers do) gives 0.5 (16 quads per 32
  * samples), so the axis march's texture roof is ctfp_sampler_peak
  * (CTFP_SAMPLER_LAYERED) x 0.5 / quad_gathers_per_sample voxel-samples/s.
- * Does not depend on the volumes.  (A plan of four materials loads its corners
+ * Does not depend on the volumes.  Counted for one thread per ray, also where
+ * the plan's forward shares rays among lanes.  (A plan of four materials loads its corners
  * without the texture unit; the count is then that of the same reuse by
  * gathers.)  No counterpart in the reference. */
 ctfp_status ctfp_axis_gather_count(ctfp_plan* plan, double* quad_gathers_per_sample);

@@ -28,18 +28,3 @@ def test_few_rows_vs_oracle(cuda_ok, V, M, mode):
         # trilinear: FP32 sums of some 1e4 terms of both signs; texture emulation: weights of
         # 1/256 steps, some of which FP32 coordinates put on the other side of a step
         assert np.max(np.abs(a - ref[m])) <= (1e-5 if mode == "trilinear" else 1e-3) * np.max(np.abs(ref[m]))
-
-
-@pytest.mark.parametrize("M", [3, 4])
-def test_more_view_groups_than_one_launch_holds(cuda_ok, M):
-    """Six parts of 15 000 views and more, one band of rows: 90 000 groups."""
-    views = 90002
-    d = small_geometry(n=4, views=views, U=2, V=2, length=4.0)
-    gL = np.random.RandomState(4).normal(size=(views * 4, M)).astype(np.float32)
-    with Projector(d, M, "trilinear") as pr:
-        pr.set_launch_shape(32, 1, 1, 2)
-        g = pr.line_integrals_adjoint(torch.from_numpy(gL.reshape(views, 2, 2, M)).cuda())
-        torch.cuda.synchronize()
-    ref = O.line_integrals_adjoint(d, gL, M, O.TRILINEAR)
-    for m in range(M):
-        assert np.max(np.abs(g[m].double().cpu().numpy() - ref[m])) <= 1e-5 * np.max(np.abs(ref[m]))
