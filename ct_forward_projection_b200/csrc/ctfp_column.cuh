@@ -33,8 +33,9 @@ __host__ __device__ __forceinline__ ColumnDims column_dims(int nx, int ny, int n
     d.elems = (size_t)d.sx * (size_t)(nx + 2 * kColPad);
     return d;
 }
-// Whether 32-bit elements reach the whole set (a volume of over 1.4e9 voxels
-// with an extent below 5 may not fit; every other one does).
+// Whether 32-bit elements reach the whole set.  Every volume of the axis sampler
+// fits; others of under 2^31 voxels may not where two extents are small (1 x 1 x
+// 172 000 000, 5 x 5 x 53 100 000) or one is and the others are long (32768 x 26240 x 1).
 __host__ __device__ __forceinline__ bool column_fits(int nx, int ny, int nz)
 {
     return (double)(nx + 2 * kColPad) * (ny + 2 * kColPad) * (nz + 2 * kColPad) < 4294967040.0;
@@ -123,9 +124,9 @@ __device__ __forceinline__ RaySeg column_segment(const GeomParams& g, int p, int
 // elements of the four materials side by side, instead of two layered texture
 // copies of each.  A footprint's voxel is then one load for all materials,
 // where the gathers cost the texture unit their time once per material: 48
-// views of 512^3, 218 -> 145 ms (texture returns 90 % busy before).  For fewer
+// views of 512^3, 219 -> 151 ms (texture returns 90 % busy before).  For fewer
 // materials the loads' lines cost the L1 as much as the gathers: 256^3, 90
-// views, 2 materials 11.9 against 12.1 ms, 3 materials 13.5 against 11.5.
+// views, 2 materials 11.9 against 12.1 ms, 3 materials 14.1 against 12.1.
 __host__ __device__ constexpr bool uses_columns(int M) { return M == 4; }
 
 // The sums of one ray over the column copy (or of its part-th of parts equal runs

@@ -496,9 +496,10 @@ __device__ __forceinline__ void kahan_join(float& s, float& c, float s2, float c
 // With a plain [E][V][U] table a warp of 4 columns loaded 16 bytes of each of 8
 // rows per energy.  Measured, plain table -> blocks: 128^3, 1 material, 61
 // energies, forward 2.107 -> 1.996 ms; 256^3, 101 energies, 2 materials, forward
-// 48.27 -> 47.9 ms, 3 materials, training step 29.7 -> 28.7 ms.  The last E % 4
+// 48.3 -> 48.1 ms, 3 materials, training step 29.7 -> 28.7 ms.  The last E % 4
 // energies are not padded to a group (one energy would take four times its
-// bytes): element (e, v, u) is float block * 32 E + 128 (e / 4) + 4 lane + e % 4,
+// bytes; the second address costs the march two registers: 128^3 2.00 -> 2.03 ms,
+// 256^3 47.9 -> 48.2): element (e, v, u) is float block * 32 E + 128 (e / 4) + 4 lane + e % 4,
 // and from e = 4 (E / 4) on block * 32 E + 32 e + lane.
 __host__ __device__ __forceinline__ int energy_groups(int E) { return (E + 3) >> 2; }
 __host__ __device__ __forceinline__ size_t weight_floats(int U, int V, int E)
